@@ -117,10 +117,10 @@ void Batch::finalize(cudaStream_t stream) {
     }
     std::vector<uint2> dec, row, crt, crt_tc, dec_tc[kMaxLogN1 + 1];
     std::vector<uint2> row_by_size[kBatchRowLogMax + 1];
-    std::vector<uint2> crt_tc32, dec_tc32[kMaxLogN1 + 1], row32_by_size[kBatchRowLogMax + 1],
+    std::vector<uint2> crt_tc32[kMaxLogN1 + 1], dec_tc32[kMaxLogN1 + 1], row32_by_size[kBatchRowLogMax + 1],
         row32_tail[kBatchRowLogMax + 1];
     kmax32_ = 1;
-    lw_tc32_ = 2;
+    for (int& lw : lw_tc32_) lw = 2;
     direct_.clear();
     int lw_tc = 2;
     size_t off = 0;
@@ -199,10 +199,12 @@ void Batch::finalize(cudaStream_t stream) {
                 // after every product's pairs, so that the pairs stay aligned to even positions
                 for (uint32_t i = 0; i < bp.n_row; ++i) row32_tail[cfg.logN2].push_back(make_uint2((kItemRow << 28) | pid, i));
             }
-            if (e.mode != kModeForward)
-                for (uint32_t i = 0; i < uint32_t(g32.tiles); ++i) crt_tc32.push_back(make_uint2(pid, i));
+            if (e.mode != kModeForward) {
+                const uint32_t tiles = 1u << (pl->logN - crt32_batch_log_tile(pl->logN));
+                for (uint32_t i = 0; i < tiles; ++i) crt_tc32[g32.logN1].push_back(make_uint2(pid, i));
+                lw_tc32_[g32.logN1] = std::max(lw_tc32_[g32.logN1], int(dw.LW));
+            }
             kmax32_ = std::max(kmax32_, pl->k32);
-            lw_tc32_ = std::max(lw_tc32_, int(dw.LW));
             shape.push_back((uint64_t(1) << 61) | (uint64_t(pl->logN) << 40) | (uint64_t(pl->k32) << 32) |
                             (uint64_t(pl->L) << 8) | e.mode);
             continue;
@@ -273,17 +275,20 @@ void Batch::finalize(cudaStream_t stream) {
         items.insert(items.end(), row32_by_size[l].begin(), row32_by_size[l].end());
         shape.push_back((uint64_t(5) << 60) | (uint64_t(l) << 32) | uint64_t(row32_by_size[l].size()));
     }
-    n_crt_tc32_ = int(crt_tc32.size());
     crt32_first_ = int(items.size());
-    items.insert(items.end(), crt_tc32.begin(), crt_tc32.end());
+    for (int l = 0; l <= kMaxLogN1; ++l) {
+        n_crt_tc32_[l] = int(crt_tc32[l].size());
+        items.insert(items.end(), crt_tc32[l].begin(), crt_tc32[l].end());
+        shape.push_back((uint64_t(4) << 60) | (uint64_t(l) << 40) | (uint64_t(lw_tc32_[l]) << 32) |
+                        uint64_t(n_crt_tc32_[l]));
+    }
     dec32_first_ = int(items.size());
     for (int l = 0; l <= kMaxLogN1; ++l) {
         n_dec_tc32_[l] = int(dec_tc32[l].size());
         items.insert(items.end(), dec_tc32[l].begin(), dec_tc32[l].end());
         shape.push_back((uint64_t(6) << 60) | (uint64_t(l) << 32) | uint64_t(n_dec_tc32_[l]));
     }
-    shape.push_back((uint64_t(7) << 60) | (uint64_t(kmax32_) << 32) | (uint64_t(lw_tc32_) << 16) |
-                    uint64_t(n_crt_tc32_));
+    shape.push_back((uint64_t(7) << 60) | (uint64_t(kmax32_) << 32));
 
     ensure(reinterpret_cast<char**>(&d_products_), &products_cap_, n * sizeof(BatchProduct), "batch products");
     ensure(&d_items_, &items_cap_, items.size(), "batch items");
@@ -413,11 +418,14 @@ void Batch::run(cudaStream_t stream, bool use_graph) {
             ga.head = d_state_ + 2 * n + 5 + kBatchRowLogMax + g;
             e = launch_persistent_rows32(ga, row_groups32_[g].logN2, row_groups32_[g].ctas, s);
         }
-        if (e == cudaSuccess && n_crt_tc32_ > 0) {
+        int at_crt32 = crt32_first_;
+        for (int l = 0; l <= kMaxLogN1 && e == cudaSuccess; ++l) {
+            if (n_crt_tc32_[l] == 0) continue;
             BatchCrtArgs ct = tc;
-            ct.items = d_items_ + crt32_first_;
-            ct.n_items = n_crt_tc32_;
-            e = launch_batch_crt_tc32(ct, lw_tc32_, s);
+            ct.items = d_items_ + at_crt32;
+            ct.n_items = n_crt_tc32_[l];
+            e = launch_batch_crt_tc32(ct, l, lw_tc32_[l], s);
+            at_crt32 += n_crt_tc32_[l];
         }
         if (!direct_.empty()) {
             // join the side stream back into s (also after a failed launch, so a capture ends whole)

@@ -47,7 +47,8 @@ class Batch {
                 (n_crt_ > 0 ? 1 : 0);
         for (int c : n_dec_tc_) n += c > 0 ? 1 : 0;
         for (const Direct& x : direct_) n += x.d.mode == kModeForward ? 2 : 3;
-        n += int(row_groups32_.size()) + (n_crt_tc32_ > 0 ? 1 : 0);
+        n += int(row_groups32_.size());
+        for (int c : n_crt_tc32_) n += c > 0 ? 1 : 0;
         for (int c : n_dec_tc32_) n += c > 0 ? 1 : 0;
         return n;
     }
@@ -108,13 +109,13 @@ class Batch {
     size_t smem_dec_tc_ = 0;
     // Products on the 30-bit engine (plain products of plans that use it, residue scratch from the
     // batch's arena), after the items above in d_items_: their row items by row-block size (one
-    // persistent launch each; heads after the 62-bit groups'), their CRT items, their residue items
-    // by log2 N1.
+    // persistent launch each; heads after the 62-bit groups'), their CRT items and their residue
+    // items by log2 N1.
     std::vector<RowGroup> row_groups32_;
-    int n_crt_tc32_ = 0;
+    int n_crt_tc32_[kMaxLogN1 + 1] = {}, lw_tc32_[kMaxLogN1 + 1] = {};  // and their widest LW
     int n_dec_tc32_[kMaxLogN1 + 1] = {};
     int crt32_first_ = 0, dec32_first_ = 0;  // positions in d_items_
-    int kmax32_ = 1, lw_tc32_ = 2;
+    int kmax32_ = 1;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     cudaEvent_t done_ = nullptr;  // recorded after every run

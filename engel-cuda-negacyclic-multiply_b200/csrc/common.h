@@ -121,10 +121,37 @@ struct QConst32 {
     uint32_t q[kMaxL + 2];
     uint32_t neg_m[kMaxL + 2];             // (-M) mod q, M = prod of the k primes
     uint32_t mu[4];                        // floor(2^(qbits + kBarrettT + 1) / q)
+    // one-word quotient of the tensor-core CRT (crt32_finish in k_w32.cu): a sum T < 2^17 q has
+    // floor(T / q) = umulhi(floor(T / 2^(qbits - 14)), mu1) >> 13, or one less
+    uint32_t top_byte;                     // c0 = max(0, floor((qbits - 1) / 8) - 4): bytes c0 .. c0 + 4 of T
+    int32_t top_shift;                     // qbits - 8 c0 - 14
+    uint32_t mu1;                          // floor(2^(qbits + 31) / q), below 2^32 for q > 1
+    uint32_t pad1;
+    uint64_t top_neg_m;                    // floor(((-M) mod q) / 2^(8 c0))
+    uint32_t neg_q[kMaxL + 2];             // 2^(32 (LW + 1)) - q
     uint32_t y[kMaxPrimes32];              // (M/p_i)^-1 N^-1 2^32 mod p_i (2^32: the pointwise Montgomery factor)
     uint32_t ys[kMaxPrimes32];             // floor(y 2^32 / p_i)
     uint32_t mq[kMaxPrimes32 * (kMaxL + 2)];  // (M/p_i) mod q, row stride kMaxL + 2
 };
+
+// The 30-bit engine's tensor-core CRT: 128-coefficient tiles (one MMA's M) from N = 2^15, 64 below and
+// 32 up to 2^11 while a row segment still holds eight columns: a CTA walks its primes x columns one
+// after another, so at small N more and shorter CTAs win (868 bits, a product: N = 16384 26.6 us with
+// 64 against 31.7 us with 128; N = 32768 42.5 us with 128, 43.7 us with 64, 54.9 us with 32; N = 1024
+// 16.0, 16.4 and 18.5 us with 32, 64 and 128). The table B has the 4 LW bytes of a coefficient sum and
+// 4 bytes of the quotient sum as columns; its accumulator takes a power of two of tensor-memory columns.
+constexpr int kCrt32Rows = 128;
+NC_HD constexpr int crt32_log_tile(int logN, int logN1) {
+    const int t = logN >= 15 ? 7 : logN >= 12 ? 6 : 5;
+    return logN < t ? logN : t - logN1 >= 3 ? t : logN < 7 ? logN : 7;
+}
+// In a batch, whose other products fill the SMs, always whole tiles.
+NC_HD constexpr int crt32_batch_log_tile(int logN) { return logN < 7 ? logN : 7; }
+NC_HD constexpr int crt32_cols(int LW) { return (4 * LW + 4 + 15) / 16 * 16; }
+NC_HD constexpr size_t crt32_table_bytes(int LW) { return size_t(crt32_cols(LW)) * 256; }
+NC_HD constexpr uint32_t crt32_tmem_cols(int LW) {
+    return crt32_cols(LW) <= 32 ? 32u : crt32_cols(LW) <= 64 ? 64u : crt32_cols(LW) <= 128 ? 128u : 256u;
+}
 
 // Operand f of a product (0: a, 1: b, 2..: x_more) and its residue buffer.
 NC_HD inline const uint32_t* factor_limbs(const ProductDesc& d, int f) {

@@ -287,25 +287,6 @@ std::vector<uint8_t> crt_tc_table(const QConst& hq) {
     return b;
 }
 
-// The same table for the 30-bit engine: K byte 4 i + a (a < 4) of output column c holds byte
-// c - a of (M/p_i) mod q.
-std::vector<uint8_t> crt_tc32_table(const QConst32& hq) {
-    const int LW = int(hq.LW), L = int(hq.L), k = int(hq.k);
-    const int NC = crt_tc_cols(LW);
-    std::vector<uint8_t> b(crt_tc_table_bytes(LW), 0);
-    for (int c = 0; c < NC; ++c)
-        for (int i = 0; i < k; ++i)
-            for (int a = 0; a < 4; ++a) {
-                const int byte = c - a;
-                if (byte < 0 || byte >= 4 * L) continue;
-                const uint32_t word = hq.mq[size_t(i) * kMqStride + size_t(byte / 4)];
-                const int K = 4 * i + a;
-                b[size_t(c / 8) * 2048 + size_t(K / 16) * 128 + size_t(c % 8) * 16 + size_t(K % 16)] =
-                    uint8_t(word >> (8 * (byte % 4)));
-            }
-    return b;
-}
-
 bool word64_forced() {
     const char* word = std::getenv("NC_WORD_BITS");
     return word && std::atoi(word) == 64;
@@ -394,7 +375,7 @@ Plan* plan_create(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int fac
             check(cudaMalloc(&p->d_qc32, sizeof(QConst32)), "30-bit plan constants");
             check(cudaMemcpyAsync(p->d_qc32, &p->hq32, sizeof(QConst32), cudaMemcpyHostToDevice, p->stream),
                   "30-bit plan constants upload");
-            crt_b32 = crt_tc32_table(p->hq32);
+            crt_b32 = crt32_table(p->hq32);
             check(cudaMalloc(&p->d_crt_b32, crt_b32.size()), "30-bit CRT table");
             check(cudaMemcpyAsync(p->d_crt_b32, crt_b32.data(), crt_b32.size(), cudaMemcpyHostToDevice, p->stream),
                   "30-bit CRT table upload");

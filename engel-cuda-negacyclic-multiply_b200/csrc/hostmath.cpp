@@ -134,19 +134,70 @@ void sub_shifted(Big& a, const Big& b, int shift) {
     trim(a);
 }
 
-// a mod m and (optionally) floor(a / m), by shift-and-subtract.
+// a mod m and (optionally) floor(a / m), m > 0: long division by 32-bit words (each quotient word
+// estimated from the three leading words of the rest and the two of m, scaled so that m's top bit
+// is set, and corrected; Knuth, The Art of Computer Programming 2, 4.3.1, algorithm D).
 Big divmod(Big a, const Big& m, Big* quot) {
     trim(a);
-    const int mb = bits_of(m);
-    int ab = bits_of(a);
-    Big q;
-    if (quot) q.assign(a.size() + 1, 0);
-    for (int shift = ab - mb; shift >= 0; --shift) {
-        if (cmp_shifted(a, m, shift) >= 0) {
-            sub_shifted(a, m, shift);
-            if (quot) q[shift >> 5] |= 1u << (shift & 31);
-        }
+    Big d = m;
+    trim(d);
+    if (quot) quot->clear();
+    if (a.size() < d.size()) return a;
+    if (d.size() == 1) {
+        uint64_t rem = 0;
+        const Big q = div_u64(a, d[0], &rem);
+        if (quot) *quot = q;
+        Big r{uint32_t(rem)};
+        trim(r);
+        return r;
     }
+    const int sh = __builtin_clz(d.back());
+    auto scale = [sh](Big& x) {  // x <<= sh, one word longer
+        x.push_back(0);
+        if (sh)
+            for (size_t i = x.size() - 1; i > 0; --i) x[i] = (x[i] << sh) | (x[i - 1] >> (32 - sh));
+        if (sh) x[0] <<= sh;
+    };
+    scale(a);
+    scale(d);
+    d.pop_back();
+    const size_t n = d.size(), top = a.size() - n;
+    Big q(top, 0);
+    for (size_t j = top; j-- > 0;) {
+        const uint64_t num = (uint64_t(a[j + n]) << 32) | a[j + n - 1];
+        uint64_t est = a[j + n] >= d[n - 1] ? 0xffffffffull : num / d[n - 1];
+        uint64_t rest = num - est * d[n - 1];
+        while (rest >> 32 == 0 && est * d[n - 2] > ((rest << 32) | a[j + n - 2])) {
+            --est;
+            rest += d[n - 1];
+        }
+        uint64_t carry = 0;
+        int64_t borrow = 0;
+        for (size_t i = 0; i < n; ++i) {
+            carry += est * d[i];
+            const int64_t t = int64_t(a[i + j]) - int64_t(uint32_t(carry)) - borrow;
+            a[i + j] = uint32_t(t);
+            borrow = t < 0 ? 1 : 0;
+            carry >>= 32;
+        }
+        const int64_t t = int64_t(a[j + n]) - int64_t(carry) - borrow;
+        a[j + n] = uint32_t(t);
+        if (t < 0) {  // one too many: add m back
+            --est;
+            uint64_t c = 0;
+            for (size_t i = 0; i < n; ++i) {
+                c += uint64_t(a[i + j]) + d[i];
+                a[i + j] = uint32_t(c);
+                c >>= 32;
+            }
+            a[j + n] += uint32_t(c);
+        }
+        q[j] = uint32_t(est);
+    }
+    a.resize(n);
+    if (sh)
+        for (size_t i = 0; i < n; ++i) a[i] = (a[i] >> sh) | (i + 1 < n ? a[i + 1] << (32 - sh) : 0);
+    trim(a);
     if (quot) {
         trim(q);
         *quot = q;
@@ -635,7 +686,49 @@ std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out) {
     divmod(pow2(qbits + kBarrettT + 1), qb, &mu);
     if (bits_of(mu) > 96) return "internal: Barrett constant too wide";
     for (size_t l = 0; l < mu.size() && l < 4; ++l) out->mu[l] = mu[l];
+    const int c0 = std::max(0, (qbits - 1) / 8 - 4);
+    out->top_byte = uint32_t(c0);
+    out->top_shift = qbits - 8 * c0 - 14;
+    Big mu1;
+    divmod(pow2(qbits + 31), qb, &mu1);
+    out->mu1 = mu1.size() > 1 ? 0xffffffffu : mu1[0];  // q = 1: every sum is zero
+    for (int b = 0; b < 5; ++b) {
+        const int byte = c0 + b;
+        out->top_neg_m |= uint64_t((out->neg_m[byte / 4] >> (8 * (byte % 4))) & 0xffu) << (8 * b);
+    }
+    uint64_t borrow = 0;
+    for (int l = 0; l <= int(out->LW); ++l) {
+        const uint64_t t = uint64_t(0) - out->q[l] - borrow;
+        out->neg_q[l] = uint32_t(t);
+        borrow = (t >> 32) ? 1 : 0;
+    }
     return std::string();
+}
+
+std::vector<uint8_t> crt32_table(const QConst32& c) {
+    const int LW = int(c.LW), L = int(c.L), k = int(c.k), NC = crt32_cols(LW);
+    const auto& ps = prime_set32();
+    Big qb(c.q, c.q + L);
+    trim(qb);
+    std::vector<uint8_t> b(crt32_table_bytes(LW), 0);
+    for (int i = 0; i < k; ++i) {
+        const uint64_t p = ps[size_t(i)].p;
+        Big mq(c.mq + size_t(i) * kMqStride, c.mq + size_t(i) * kMqStride + kMqStride);
+        trim(mq);
+        for (int a = 0; a < 4; ++a) {
+            const uint64_t w = (uint64_t(c.y[i]) << (8 * a)) % p;
+            Big e = divmod(mul_u64(mq, w), qb, nullptr);
+            e.resize(size_t(LW), 0);
+            const uint32_t phi = uint32_t((w << 32) / p);
+            const int K = 4 * i + a;
+            for (int col = 0; col < 4 * LW + 4 && col < NC; ++col) {
+                const uint32_t word = col < 4 * LW ? e[size_t(col / 4)] : phi;
+                b[size_t(col / 8) * 2048 + size_t(K / 16) * 128 + size_t(col % 8) * 16 + size_t(K % 16)] =
+                    uint8_t(word >> (8 * (col % 4)));
+            }
+        }
+    }
+    return b;
 }
 
 std::string check_qconst32(const QConst32& c) {
@@ -668,6 +761,16 @@ std::string check_qconst32(const QConst32& c) {
     trim(mu);
     const Big e = pow2(int(c.qbits) + kBarrettT + 1);
     if (cmp_big(mul_big(mu, qb), e) > 0 || cmp_big(add_big(mul_big(mu, qb), qb), e) <= 0) return "Barrett constant mu";
+    Big m1{c.mu1};
+    const Big e1 = pow2(int(c.qbits) + 31);
+    if (bits_of(qb) > 1 && (cmp_big(mul_big(m1, qb), e1) > 0 || cmp_big(add_big(mul_big(m1, qb), qb), e1) <= 0))
+        return "one-word quotient constant";
+    uint64_t carry = 0;
+    for (int l = 0; l <= int(c.LW); ++l) {
+        carry += uint64_t(c.neg_q[l]) + c.q[l];
+        if (uint32_t(carry) != 0) return "two's complement of q";
+        carry >>= 32;
+    }
     return std::string();
 }
 

@@ -65,6 +65,12 @@ int primes_needed32(int logN, int qbits);
 // The 30-bit engine's CRT + Barrett constants. Returns an empty string or an error message.
 std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out);
 
+// Table B of the 30-bit engine's tensor-core CRT in the MMA's shared-memory order. K byte 4 i + a
+// (byte a of residue r_i) has weight E = (2^(8a) y_i mod p_i) (M/p_i) mod q: columns c < 4 LW hold
+// byte c of E, columns 4 LW .. 4 LW + 3 the bytes of floor(2^32 (2^(8a) y_i mod p_i) / p_i), the
+// term's share of the quotient; at (c / 8) * 2048 + (K / 16) * 128 + (c % 8) * 16 + K % 16.
+std::vector<uint8_t> crt32_table(const QConst32& c);
+
 std::string check_prime_set32();                                 // primes, 1 mod 2^17, constants
 std::string check_tables32(const HostTables32& t, int samples);  // psi, 2^(32 l) mod p, twiddles
 std::string check_qconst32(const QConst32& c);                   // CRT identities and mu

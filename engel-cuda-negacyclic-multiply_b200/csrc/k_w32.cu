@@ -8,8 +8,8 @@
 // one pass of MMAs (128 accumulator columns) covers 32 primes. The folded sum (< 2^48) is reduced
 // with one multiply by floor(2^50 / p).
 //
-// CRT. v_i = r_i y_i mod p_i < 2^30 is 4 bytes, so A has K = 4 k <= 256 bytes and the table B has
-// B[c][4 i + a] = byte c - a of (M/p_i) mod q; every S_c < 4 k 255^2 < 2^24.
+// CRT. The 4 bytes of each residue against a per-plan table (K = 4 k <= 256 bytes) that carries the
+// factors y_i, the reduction of M/p_i mod q and the quotient (below, at the CRT's kernels).
 #include "batch_types.h"
 #include "crt_tc.cuh"
 #include "kernel_registry.h"
@@ -21,7 +21,6 @@ namespace w32 {
 
 namespace {
 
-using crt_tc_detail::a_offset;
 using crt_tc_detail::kmajor_desc;
 using crt_tc_detail::mma_wait;
 using crt_tc_detail::smem_u32;
@@ -271,256 +270,386 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
 }
 
 // ------------------------------------------------------------------------------------------
-// CRT: inverse column stages, v_i = r_i y_i mod p_i into A (4 bytes at K offset 4 i), the
-// contraction, the quotient estimate and Barrett (crt_coeffs_tc of crt_tc.cuh on 30-bit residues)
+// CRT: inverse column stages into A (the raw residues' 4 bytes at K offset 4 i), the contraction
+// with the plan's table (crt32_table, hostmath.h) and the one-word quotient.
+//
+// With r_i in [0, 2p_i) the residue of the transform (still to be multiplied by y_i), byte a of
+// r_i has the weight E_{i,a} = (2^(8a) y_i mod p_i) (M/p_i), so x = sum r_{i,a} E_{i,a} - K M with
+// K = round(sum r_{i,a} phi_{i,a}), phi = (2^(8a) y_i mod p_i) / p_i: the table holds E mod q and
+// phi, so neither the product r_i y_i nor a separate quotient sum is left to the integer pipes. The
+// byte sums are below 4 * 64 * 255^2 < 2^24; K is exact because |x| < M / 8 and the floors of 256
+// terms lose less than 255 * 256 / 2^32 (phi has 32 bits); and T = sum r_{i,a} (E mod q) +
+// K ((-M) mod q) < 2^17 q, whose quotient by q is one word.
+//
+// What bounds it: the column butterflies and loads (59 residues of a coefficient against one
+// contraction row), so integer issue and load latency, not the tensor cores. 128-coefficient tiles
+// with the primes in passes of 32 through one 16 KB A buffer keep a CTA at 49 KB, four per SM.
 
-template <int LOG_N1>
-__device__ void crt32_columns(const ProductDesc& d, const Tables& t, int j0, int T, const uint32_t* s_y,
-                              const uint32_t* s_ys, const uint32_t* s_p, uint8_t* sA) {
+// Byte offset of (row, prime il of the pass) in A: [16 row groups][8 K chunks][8 rows][16 B].
+__device__ __forceinline__ int crt32_at(int row, int il) {
+    return (row >> 3) * 1024 + (il >> 2) * 128 + (row & 7) * 16 + (il & 3) * 4;
+}
+
+// Primes [i0, i0 + np) of the tile's 2^logC columns: N1 residues at stride N2 (2^LN2, or N / N1 with
+// LN2 0), the inverse stages of the merged tree, four bytes each into A. Items (prime, column) with
+// eight columns of four primes to a warp: its loads are whole sectors and its four-byte stores fall
+// on 32 banks. Both strides are loop constants (rows u C + j with C >= 8 are C * 128 bytes apart in
+// A): 18 multiply-adds a residue went to addresses before. Short columns (N1 <= 4) are loaded
+// several items at a time: one load after another would be the stage's whole time at small N.
+template <int LOG_N1, int LN2>
+__device__ __forceinline__ void crt32_columns(const uint32_t* res, const uint2* tw0, int logN, int logC, int np,
+                                           const uint32_t* s_p, uint8_t* sA) {
     constexpr int N1 = 1 << LOG_N1;
-    const int N = 1 << d.logN;
-    const int N2 = N >> LOG_N1;
-    const int C = T >> LOG_N1;
-    const int k = int(d.k);
-    const uint32_t* res = reinterpret_cast<const uint32_t*>(d.ra);
-    auto put = [&](int tc, int i, uint32_t v) {
-        *reinterpret_cast<uint32_t*>(sA + (tc >> 7) * kCrtTcHalfBytes + a_offset(tc & 127, 4 * i)) = v;
-    };
+    const int N = 1 << logN;
+    const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
+    const int C = 1 << logC;
+    const int tid = int(threadIdx.x);
     if constexpr (LOG_N1 == 5) {
         // 32-point columns on two adjacent lanes (as crt_columns_tc): lane h loads rows
         // [16h, 16h + 16), runs the inverse stages of its half-subtree, and the last stage's pairs
         // (u, u + 16) are split between the lanes after one exchange of eight values
-        const int total = 2 * k * C;
-        const int lane = int(threadIdx.x) & 31;
-        for (int w0 = int(threadIdx.x) & ~31; w0 < total; w0 += int(blockDim.x)) {
+        const int total = 2 * np * C;
+        const int lane = tid & 31;
+        for (int w0 = tid & ~31; w0 < total; w0 += kThreads) {
             const int w = w0 + lane;
             const bool active = w < total;
             const int item = active ? w >> 1 : 0, h = w & 1;
-            const int i = item / C, j = item - i * C;
-            const uint32_t* row = res + size_t(i) * N + j0 + j + size_t(16 * h) * N2;
+            const int i = item >> logC, j = item & (C - 1);
+            const uint32_t* row = res + size_t(i) * N + j + size_t(16 * h) * N2;
             uint32_t v[16];
 #pragma unroll
             for (int u = 0; u < 16; ++u) v[u] = active ? __ldcg(row + size_t(u) * N2) : 0u;
             const uint32_t p = s_p[i], p2 = 2 * p;
-            const uint2* tw = t.inv32 + size_t(i) * kMaxN;
+            const uint2* tw = tw0 + size_t(i) * kMaxN;
             w32::column_inverse_root<4>(tw, 2 + h, p, v);
             const uint2 w1 = __ldg(tw + 1);
-            const uint32_t y = s_y[i], ys = s_ys[i];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? v[e] : v[8 + e], 1);
                 uint32_t lo = h ? got : v[e], hi = h ? v[8 + e] : got;  // rows 8h + e and 8h + e + 16
                 w32::gs_bfly(lo, hi, w1.x, w1.y, p, p2);
                 if (active) {
-                    put((8 * h + e) * C + j, i, w32::csub(w32::shoup(lo, y, ys, p), p));
-                    put((8 * h + e + 16) * C + j, i, w32::csub(w32::shoup(hi, y, ys, p), p));
+                    *reinterpret_cast<uint32_t*>(sA + crt32_at((8 * h + e) * C + j, i)) = lo;
+                    *reinterpret_cast<uint32_t*>(sA + crt32_at((8 * h + e + 16) * C + j, i)) = hi;
                 }
             }
         }
     } else {
-        for (int w = threadIdx.x; w < k * C; w += blockDim.x) {
-            const int i = w / C, j = w - i * C;
-            const uint32_t* row = res + size_t(i) * N + j0 + j;
-            uint32_t v[N1];
+        constexpr int U = LOG_N1 >= 3 ? 1 : 8 >> LOG_N1;  // items in flight per thread
+        const bool wide = logC >= 3;
+        const int total = (wide ? (np + 3) & ~3 : np) << logC;
+        auto split = [&](int w, int& i, int& j) {
+            if (wide) {
+                const int hi = w >> 5;
+                i = ((hi >> (logC - 3)) << 2) + ((w >> 3) & 3);
+                j = ((hi & ((C >> 3) - 1)) << 3) + (w & 7);
+            } else {
+                i = w >> logC;
+                j = w & (C - 1);
+            }
+        };
+#pragma unroll 1
+        for (int w0 = tid; w0 < total; w0 += kThreads * U) {
+            uint32_t v[U][N1];
 #pragma unroll
-            for (int u = 0; u < N1; ++u) v[u] = __ldcg(row + size_t(u) * N2);
-            const uint32_t p = s_p[i];
-            if (LOG_N1 > 0) w32::column_inverse_root<LOG_N1>(t.inv32 + size_t(i) * kMaxN, 1, p, v);
-            const uint32_t y = s_y[i], ys = s_ys[i];
+            for (int q = 0; q < U; ++q) {
+                int i, j;
+                split(w0 + q * kThreads, i, j);
+                const bool active = w0 + q * kThreads < total && i < np;
+                const uint32_t* row = res + (active ? size_t(i) * N + j : size_t(0));
 #pragma unroll
-            for (int u = 0; u < N1; ++u) put(u * C + j, i, w32::csub(w32::shoup(v[u], y, ys, p), p));
+                for (int u = 0; u < N1; ++u) v[q][u] = __ldcg(row + size_t(u) * N2);
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                int i, j;
+                split(w0 + q * kThreads, i, j);
+                if (w0 + q * kThreads < total && i < np) {
+                    if (LOG_N1 > 0) w32::column_inverse_root<LOG_N1>(tw0 + size_t(i) * kMaxN, 1, s_p[i], v[q]);
+                    if (wide) {
+                        uint8_t* at = sA + crt32_at(j, i);
+#pragma unroll
+                        for (int u = 0; u < N1; ++u) *reinterpret_cast<uint32_t*>(at + (u << logC) * 128) = v[q][u];
+                    } else {
+#pragma unroll
+                        for (int u = 0; u < N1; ++u) *reinterpret_cast<uint32_t*>(sA + crt32_at(u * C + j, i)) = v[q][u];
+                    }
+                }
+            }
         }
     }
 }
 
-// Shared memory of the 30-bit CRT: A (two halves of 128 rows x 256 K bytes), the plan's table,
-// y, its companion and p of up to 64 primes, (-M) mod q, q and mu; raised so that no more CTAs
-// share an SM than its tensor memory holds (as crt_tc_smem_bytes).
-NC_HD constexpr size_t crt_tc32_smem_bytes(int LW) {
-    return smax(size_t(2) * kCrtTcHalfBytes + crt_tc_table_bytes(LW) + size_t(kMaxPrimes32) * 4 * 3 +
-                    size_t(kMqStride) * 4 * 2 + 16 + 16,
-                (size_t(233472) / (512 / crt_tc_tmem_cols(LW) + 1) + 16) / 16 * 16);
+__device__ __forceinline__ void tmem_ld4(uint32_t (&s)[4], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t (&s)[8], uint32_t addr) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// Constants of the finish in shared memory, each padded to whole 16-byte words.
+constexpr int kCrt32Words = 36;
+
+// This thread's coefficient from its lane of the accumulator, T mod q, to L limbs at `o` (if `store`).
+// All the lanes of a warp together (tensor-memory loads). Not inlined: one copy for each LW serves the
+// kernels of every column length, and at its call nothing of theirs is live.
+template <int LW>
+__device__ __noinline__ void crt32_finish(const QConst32* qc, const uint32_t* s_negm, const uint32_t* s_nq,
+                                          const uint32_t* s_q, uint32_t lane_base, int L, uint32_t* o, bool store) {
+    uint32_t r[LW + 1];
+    const int c0 = int(__ldg(&qc->top_byte)), sh = __ldg(&qc->top_shift);
+    uint32_t ph[4], top[8];
+    tmem_ld4(ph, lane_base + uint32_t(4 * LW));
+    tmem_ld8(top, lane_base + uint32_t(c0));
+    tmem_wait_ld();
+    const uint64_t phi = mad_wide(ph[3], 1u << 24, mad_wide(ph[2], 1u << 16, mad_wide(ph[1], 1u << 8, uint64_t(ph[0]))));
+    const uint32_t kq = uint32_t((phi + (1ull << 31)) >> 32);
+    // bytes c0 .. c0 + 4 of T (the bytes below add less than 2^18 units of 2^(8 c0), against
+    // q >= 2^(32 + 8 c0) where c0 > 0), then its 31 leading bits
+    uint64_t vt = mad_wide(top[3], 1u << 24, mad_wide(top[2], 1u << 16, mad_wide(top[1], 1u << 8, uint64_t(top[0])))) +
+                  (uint64_t(top[4]) << 32);
+    vt += uint64_t(kq) * __ldg(&qc->top_neg_m);
+    const uint32_t y = uint32_t(sh >= 0 ? vt >> sh : vt << -sh);
+    const uint32_t qh = __umulhi(y, __ldg(&qc->mu1)) >> 13;  // floor(T / q) or one less
+    // T - qh q = sum of bytes + kq ((-M) mod q) + qh (2^(32 (LW + 1)) - q), one carry pass; the next
+    // columns are on their way while two words are formed
+    uint64_t carry = 0;
+    uint32_t s[2][8];
+    tmem_ld8(s[0], lane_base);
+    tmem_wait_ld();
+#pragma unroll
+    for (int g = 0; g < LW / 2; ++g) {
+        if (g + 1 < LW / 2) tmem_ld8(s[(g + 1) & 1], lane_base + uint32_t(8 * (g + 1)));
+        const uint32_t* sg = s[g & 1];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int w = 2 * g + e;
+            const uint32_t lo = sg[4 * e] + (sg[4 * e + 1] << 8), hi = sg[4 * e + 2] + (sg[4 * e + 3] << 8);
+            const uint64_t own = mad_wide(hi, 1u << 16, mad_wide(qh, s_nq[w], mad_wide(kq, s_negm[w], uint64_t(lo))));
+            carry += own;
+            r[w] = uint32_t(carry);
+            carry >>= 32;
+        }
+        if (g + 1 < LW / 2) tmem_wait_ld();
+    }
+    r[LW] = uint32_t(mad_wide(qh, 0xffffffffu, carry));
+    // r < 2q: the leading two words decide, except for about one coefficient in 2^12
+    const uint64_t rt = (uint64_t(r[LW - 1]) << 32) | r[LW - 2], qt = (uint64_t(s_q[LW - 1]) << 32) | s_q[LW - 2];
+    if (r[LW] != 0 || rt >= qt) {
+        uint32_t b = 0;
+#pragma unroll
+        for (int w = 0; w < LW; ++w) {
+            const uint64_t df = uint64_t(r[w]) - s_q[w] - b;
+            b = uint32_t(df >> 32) & 1u;
+        }
+        if (r[LW] >= b) {
+            b = 0;
+#pragma unroll
+            for (int w = 0; w < LW; ++w) {
+                const uint64_t df = uint64_t(r[w]) - s_q[w] - b;
+                r[w] = uint32_t(df);
+                b = uint32_t(df >> 32) & 1u;
+            }
+        }
+    }
+    if (!store) {
+        // rows beyond a tile of fewer than 32
+    } else if ((L & 3) == 0) {
+#pragma unroll
+        for (int l = 0; l < LW; l += 4)
+            if (l < L) *reinterpret_cast<uint4*>(o + l) = make_uint4(r[l], r[l + 1], r[l + 2], r[l + 3]);
+    } else if ((L & 1) == 0) {
+#pragma unroll
+        for (int l = 0; l < LW; l += 2)
+            if (l < L) *reinterpret_cast<uint2*>(o + l) = make_uint2(r[l], r[l + 1]);
+    } else {
+#pragma unroll
+        for (int l = 0; l < LW; ++l)
+            if (l < L) o[l] = r[l];
+    }
 }
 
+// The same coefficient (row u, column j) on the integer pipes, for a tile whose MMAs did not report
+// completion in time: the column sum from its definition, x_u N1 = sum_u' z_u' rho_u'^-2u with rho_u'
+// the forward twiddle of row block u' (node N1 + u'), then v_i = r_i y_i and the carry chains.
 template <int LW>
-__device__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, uint8_t* smem, uint32_t taddr,
-                                uint64_t* bar, uint32_t parity) {
+__device__ __noinline__ void crt32_coeff_plain(const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
+                                               const uint2* inv, int logN, int logN1, int k, int L, int u, int j,
+                                               uint32_t* out) {
     constexpr int W = LW + kAccExtra;
-    constexpr int NC = crt_tc_cols(LW);
-    constexpr uint32_t kHalfCol = crt_tc_tmem_cols(LW) / 2;
+    const int N = 1 << logN, N2 = N >> logN1;
+    uint32_t acc[W], acc_hi[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) acc[w] = acc_hi[w] = 0;
+    uint64_t frac = 0;
+#pragma unroll 1
+    for (int i = 0; i < k; ++i) {
+        const uint64_t p = __ldg(&pc[i].p);
+        uint64_t x = 0;
+        for (int u2 = 0; u2 < (1 << logN1); ++u2) {
+            const uint64_t z = __ldcg(res + size_t(i) * N + size_t(u2) * N2 + j);
+            const uint64_t rho = __ldg(&inv[size_t(i) * kMaxN + (1 << logN1) + u2].x);
+            const uint64_t step = rho * rho % p;
+            uint64_t w = 1;
+            for (int e = 0; e < u; ++e) w = w * step % p;
+            x = (x + z * w) % p;
+        }
+        const uint32_t v = uint32_t(x * __ldg(qc->y + i) % p);
+        frac += (uint64_t(v) * __ldg(&pc[i].quo)) >> 29;
+        const uint32_t* M = qc->mq + i * kMqStride;
+        uint32_t m[LW];
+#pragma unroll
+        for (int l = 0; l < LW; ++l) m[l] = __ldg(M + l);
+        mac_lo<LW, 0, W>(acc, m, v);
+        mac_hi<LW, 1, W>(acc_hi, m, v);
+    }
+    mac_lo<LW, 0, W>(acc, qc->neg_m, uint32_t((frac + (1ull << 31)) >> 32));
+    mac_hi<LW, 1, W>(acc_hi, qc->neg_m, uint32_t((frac + (1ull << 31)) >> 32));
+    asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(acc_hi[0]));
+#pragma unroll
+    for (int w = 1; w < W - 1; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[w]) : "r"(acc_hi[w]));
+    asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[W - 1]) : "r"(acc_hi[W - 1]));
+    uint32_t r[LW + 1];
+    barrett<LW, W>(acc, qc->q, qc->mu, int(qc->qbits), r);
+    for (int l = 0; l < L; ++l) out[l] = r[l];
+}
+
+// Shared memory: A (128 rows x the 128 K bytes of 32 primes; the output tile once the sums are
+// out), the finish's constants, p of up to 64 primes, the plan's table; raised so that no more CTAs
+// share an SM than its tensor memory holds.
+NC_HD constexpr size_t crt_tc32_smem_bytes(int LW) {
+    return smax(size_t(kCrt32Rows) * 128 + crt32_table_bytes(LW) + size_t(kMaxPrimes32) * 4 + size_t(kCrt32Words) * 4 * 3,
+                (size_t(233472) / (512 / crt32_tmem_cols(LW) + 1) + 16) / 16 * 16);
+}
+
+// The output tile (N1 segments of C consecutive coefficients) to its place in c: a warp a segment
+// where there are as many segments as warps, else store_tile.
+__device__ __forceinline__ void crt32_store(uint32_t* c, int N2, int L, int j0, int C, int N1, const uint32_t* s_out) {
+    const int seg = C * L;
+    if (N1 < kThreads / 32 || ((size_t(N2) * L | size_t(j0) * L | size_t(seg)) & 3) != 0) {
+        store_tile(c, N2, L, j0, C, N1, s_out);
+        return;
+    }
+    const int warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
+    for (int u = warp; u < N1; u += kThreads / 32) {
+        uint4* dst = reinterpret_cast<uint4*>(c + (size_t(u) * N2 + j0) * L);
+        const uint4* src = reinterpret_cast<const uint4*>(s_out + u * seg);
+        for (int x = lane; x < (seg >> 2); x += 32) dst[x] = src[x];
+    }
+}
+
+// One tile with every thread of a 256-thread CTA, columns of 2^LOG_N1 points at stride 2^LN2 (N / N1
+// with LN2 0). The caller owns tensor-memory columns for the product's LW at `taddr` and an
+// initialised mbarrier `bar`.
+template <int LOG_N1, int LN2>
+__device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
+                                                uint8_t* smem, uint32_t taddr, uint64_t* bar) {
+    const int LW = int(d.LW), NC = crt32_cols(LW);
     const int N = 1 << d.logN;
-    const int logN1 = int(d.logN) - int(d.logN2);
-    const int N2 = N >> logN1;
-    const int T = N < kTile ? N : kTile;
-    const int C = T >> logN1;
+    const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
+    const int T = 1 << logT;
+    const int logC = logT - LOG_N1, C = 1 << logC;
     const int k = int(d.k), L = int(d.L);
     const int j0 = tile * C;
 
     uint8_t* sA = smem;
-    uint8_t* sB = smem + 2 * kCrtTcHalfBytes;
-    uint32_t* s_y = reinterpret_cast<uint32_t*>(sB + NC * 256);
-    uint32_t* s_ys = s_y + kMaxPrimes32;
-    uint32_t* s_p = s_ys + kMaxPrimes32;
-    uint32_t* s_negm = s_p + kMaxPrimes32;
-    uint32_t* s_q = s_negm + kMqStride;
-    uint32_t* s_mu = s_q + kMqStride;
+    uint32_t* s_negm = reinterpret_cast<uint32_t*>(sA + kCrt32Rows * 128);
+    uint32_t* s_nq = s_negm + kCrt32Words;
+    uint32_t* s_q = s_nq + kCrt32Words;
+    uint32_t* s_p = s_q + kCrt32Words;
+    uint8_t* sB = reinterpret_cast<uint8_t*>(s_p + kMaxPrimes32);
     const int tid = int(threadIdx.x), warp = tid >> 5;
 
-    __syncthreads();
     const QConst32* qc = d.qc32;
-    for (int w = tid; w < k; w += blockDim.x) {
-        s_y[w] = __ldg(qc->y + w);
-        s_ys[w] = __ldg(qc->ys + w);
-        s_p[w] = __ldg(&t.pc32[w].p);
-    }
-    for (int w = tid; w < kMqStride; w += blockDim.x) {
+    for (int w = tid; w < k; w += kThreads) s_p[w] = __ldg(&t.pc32[w].p);
+    for (int w = tid; w < kMqStride; w += kThreads) {
         s_negm[w] = __ldg(qc->neg_m + w);
+        s_nq[w] = __ldg(qc->neg_q + w);
         s_q[w] = __ldg(qc->q + w);
     }
-    if (tid < 4) s_mu[tid] = __ldg(qc->mu + tid);
-    // the table is first read by the MMAs: its copy runs behind the column stages (its K bytes
-    // from 4 k up to the last slice's end are zero, so A's are never read into the sums)
-    for (int w = tid; w < NC * 16; w += blockDim.x) cp_async16(sB + 16 * w, d.crt_b + w);
+    // the table is first read by the MMAs: its copy runs behind the column stages (the K chunks
+    // that the last slice reads; its K bytes from 4 k up are zero, so A's are never read into the sums)
+    const int slices_all = (4 * k + 31) / 32;
+    for (int w = tid; w < NC * 16; w += kThreads)
+        if (((w >> 3) & 15) < 2 * slices_all) cp_async16(sB + 16 * w, d.crt_b + w);
     asm volatile("cp.async.commit_group;" ::: "memory");
     __syncthreads();
     pdl_wait();  // the residues come from the stream's previous kernel
+    pdl_trigger();
 
-    switch (logN1) {
-        case 0: crt32_columns<0>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-        case 1: crt32_columns<1>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-        case 2: crt32_columns<2>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-        case 3: crt32_columns<3>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-        case 4: crt32_columns<4>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-        default: crt32_columns<5>(d, t, j0, T, s_y, s_ys, s_p, sA); break;
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-
-    if (tid == 0) {
-        const uint32_t idesc = (2u << 4) | (uint32_t(NC >> 3) << 17) | (uint32_t(128 >> 4) << 24);
-        const int slices = (4 * k + 31) / 32;
-        const uint32_t b0 = smem_u32(sB);
-        for (int h = 0; h < (T > 128 ? 2 : 1); ++h) {
-            const uint32_t a0 = smem_u32(sA + h * kCrtTcHalfBytes);
-            for (int s = 0; s < slices; ++s) {
-                const uint64_t da = kmajor_desc(a0 + uint32_t(s) * 256u, 128u, 2048u);
+    const uint32_t bar_addr = smem_u32(bar);
+    const int passes = (k + 31) >> 5;
+    bool ok = true;
+#pragma unroll 1
+    for (int g = 0; g < passes; ++g) {
+        // the A buffer is free once the pass before has been read
+        if (g > 0) ok = __syncthreads_and(ok && mma_wait(bar_addr, uint32_t((g - 1) & 1)) ? 1 : 0) != 0;
+        if (!ok) break;
+        const int i0 = 32 * g, np = k - i0 < 32 ? k - i0 : 32;
+        crt32_columns<LOG_N1, LN2>(reinterpret_cast<const uint32_t*>(d.ra) + size_t(i0) * N + j0,
+                                   t.inv32 + size_t(i0) * kMaxN, int(d.logN), logC, np, s_p + i0, sA);
+        if (g == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0) {
+            const uint32_t idesc = (2u << 4) | (uint32_t(NC >> 3) << 17) | (uint32_t(kCrt32Rows >> 4) << 24);
+            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB) + uint32_t(g) * 1024u;
+            for (int s = 0; s < (4 * np + 31) / 32; ++s) {
+                const uint64_t da = kmajor_desc(a0 + uint32_t(s) * 256u, 128u, 1024u);
                 const uint64_t db = kmajor_desc(b0 + uint32_t(s) * 256u, 128u, 2048u);
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(taddr + uint32_t(h) * kHalfCol),
-                    "l"(da), "l"(db), "r"(idesc), "r"(s));
+                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(taddr),
+                    "l"(da), "l"(db), "r"(idesc), "r"(g + s));
             }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr)
+                         : "memory");
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                     : "memory");
     }
-
-    // while the MMAs run: this thread's coefficient and the CRT quotient round(sum v_i / p_i)
-    const int tc = tid;
-    const int half = tc >> 7;
-    const uint8_t* arow = sA + half * kCrtTcHalfBytes + a_offset(tc & 127, 0);
-    uint64_t frac = 0;
-#pragma unroll 4
-    for (int i = 0; i < k; ++i) {
-        const uint32_t v = *reinterpret_cast<const uint32_t*>(arow + (i >> 2) * 128 + (i & 3) * 4);
-        frac += (uint64_t(v) * __ldg(&t.pc32[i].quo)) >> 29;  // 2^32 v / p_i, short by less than 3
-    }
-    const uint32_t kq = uint32_t((frac + (1ull << 31)) >> 32);
-
-    const bool ok = mma_wait(smem_u32(bar), parity);
+    ok = __syncthreads_and(ok && mma_wait(bar_addr, uint32_t((passes - 1) & 1)) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t acc[W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) acc[w] = 0;
-    if (__all_sync(0xffffffffu, ok)) {
-        const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(half) * kHalfCol;
-        uint64_t carry = 0;
-#pragma unroll
-        for (int cb = 0; cb < NC / 8; ++cb) {
-            uint32_t s[8];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7])
-                : "r"(lane_base + uint32_t(8 * cb)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const uint64_t t0 = carry + s[0] + (uint64_t(s[1]) << 8) + (uint64_t(s[2]) << 16) + (uint64_t(s[3]) << 24);
-            if (2 * cb < W) acc[2 * cb] = uint32_t(t0);
-            const uint64_t t1 =
-                (t0 >> 32) + s[4] + (uint64_t(s[5]) << 8) + (uint64_t(s[6]) << 16) + (uint64_t(s[7]) << 24);
-            if (2 * cb + 1 < W) acc[2 * cb + 1] = uint32_t(t1);
-            carry = t1 >> 32;
-        }
-    } else {
-        // the MMAs did not report completion in time: the same sum on the integer pipes
-        uint32_t acc_hi[W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) acc_hi[w] = 0;
-#pragma unroll 1
-        for (int i = 0; i < k; ++i) {
-            const uint32_t v = *reinterpret_cast<const uint32_t*>(arow + (i >> 2) * 128 + (i & 3) * 4);
-            const uint32_t* M = qc->mq + i * kMqStride;
-            uint32_t m[LW];
-#pragma unroll
-            for (int l = 0; l < LW; ++l) m[l] = __ldg(M + l);
-            mac_lo<LW, 0, W>(acc, m, v);
-            mac_hi<LW, 1, W>(acc_hi, m, v);
-        }
-        asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(acc_hi[0]));
-#pragma unroll
-        for (int w = 1; w < W - 1; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[w]) : "r"(acc_hi[w]));
-        asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[W - 1]) : "r"(acc_hi[W - 1]));
-    }
-    {
-        uint32_t acc_hi[W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) acc_hi[w] = 0;
-        mac_lo<LW, 0, W>(acc, s_negm, kq);
-        mac_hi<LW, 1, W>(acc_hi, s_negm, kq);
-        asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(acc_hi[0]));
-#pragma unroll
-        for (int w = 1; w < W - 1; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[w]) : "r"(acc_hi[w]));
-        asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[W - 1]) : "r"(acc_hi[W - 1]));
-    }
-    uint32_t r[LW + 1];
-    barrett<LW, W>(acc, s_q, s_mu, int(qc->qbits), r);
 
+    // every MMA has read A: it takes the output tile
+    uint32_t* s_out = reinterpret_cast<uint32_t*>(sA);
+    if (32 * warp < T) {
+        uint32_t* o = s_out + tid * L;
+        switch (LW) {
+#define NC_CRT32_FINISH(n)                                                                                     \
+    case n:                                                                                                    \
+        if (ok)                                                                                                \
+            crt32_finish<n>(qc, s_negm, s_nq, s_q, taddr + (uint32_t(32 * warp) << 16), L, o, tid < T);         \
+        else if (tid < T)                                                                                      \
+            crt32_coeff_plain<n>(reinterpret_cast<const uint32_t*>(d.ra), qc, t.pc32, t.inv32, int(d.logN),     \
+                                 LOG_N1, k, L, tid >> logC, j0 + (tid & (C - 1)), o);                          \
+        break;
+            NC_LW_CASES(NC_CRT32_FINISH)
+#undef NC_CRT32_FINISH
+            default: break;
+        }
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    uint32_t* s_out = reinterpret_cast<uint32_t*>(sA);
-    if (tc < T) {
-        uint32_t* o = s_out + tc * L;
-        if ((L & 3) == 0) {
-#pragma unroll
-            for (int l = 0; l < LW; l += 4)
-                if (l < L) *reinterpret_cast<uint4*>(o + l) = make_uint4(r[l], r[l + 1], r[l + 2], r[l + 3]);
-        } else if ((L & 1) == 0) {
-#pragma unroll
-            for (int l = 0; l < LW; l += 2)
-                if (l < L) *reinterpret_cast<uint2*>(o + l) = make_uint2(r[l], r[l + 1]);
-        } else {
-#pragma unroll
-            for (int l = 0; l < LW; ++l)
-                if (l < L) o[l] = r[l];
-        }
-    }
-    __syncthreads();
-    store_tile(d.c, N2, L, j0, C, 1 << logN1, s_out);
+    crt32_store(d.c, N2, L, j0, C, 1 << LOG_N1, s_out);
+    if (!ok) mma_wait(bar_addr, uint32_t((passes - 1) & 1));  // late MMAs end before the tensor memory is given back
 }
 
-template <int LW>
-__global__ void __launch_bounds__(kThreads, 2) k_crt_tc32(ProductDesc d, Tables t) {
-#if NC_HAS_TCGEN05
-    constexpr uint32_t kCols = crt_tc_tmem_cols(LW);
+// The tile within a kernel: tensor memory (`cols` columns) and the mbarrier around it.
+template <int LOG_N1>
+__device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t, int tile, int logT, uint32_t cols) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bar;
     __shared__ uint32_t taddr_slot;
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&taddr_slot)),
-                     "r"(kCols)
+                     "r"(cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -531,13 +660,21 @@ __global__ void __launch_bounds__(kThreads, 2) k_crt_tc32(ProductDesc d, Tables 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    pdl_trigger();  // only once the CTA holds its tensor memory
     const uint32_t taddr = taddr_slot;
-    crt32_coeffs_tc<LW>(d, t, int(blockIdx.x), smem, taddr, &bar, 0);
+    if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
+        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, smem, taddr, &bar);
+    else
+        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, smem, taddr, &bar);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+}
+
+template <int LOG_N1>
+__global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables t, int logT, uint32_t cols) {
+#if NC_HAS_TCGEN05
+    crt32_cta<LOG_N1>(d, t, int(blockIdx.x), logT, cols);
 #endif
 }
 
@@ -647,42 +784,13 @@ __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) 
     }
 }
 
-// CRT items (x = product, y = 256-coefficient tile); products of at most 30 limbs (256 columns of
-// tensor memory per CTA).
-__global__ void __launch_bounds__(kThreads, 2) k_batch_crt_tc32(BatchCrtArgs a) {
+// CRT items (x = product, y = tile) of the products with column length 2^LOG_N1.
+template <int LOG_N1>
+__global__ void __launch_bounds__(kThreads, 4) k_batch_crt_tc32(BatchCrtArgs a, uint32_t cols) {
 #if NC_HAS_TCGEN05
-    extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
-    __shared__ uint32_t taddr_slot;
-    if (threadIdx.x < 32) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;" ::"r"(smem_u32(&taddr_slot))
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    pdl_trigger();  // only once the CTA holds its tensor memory
-    const uint32_t taddr = taddr_slot;
     const uint2 w = __ldg(a.items + blockIdx.x);
-    const BatchProduct& bp = a.products[w.x];
-    switch (bp.d.LW) {
-#define NC_B_CRT_TC32(n)                                                        \
-    case n:                                                                     \
-        if constexpr (crt_tc_tmem_cols(n) == 256)                               \
-            crt32_coeffs_tc<n>(bp.d, a.tables, int(w.y), smem, taddr, &bar, 0); \
-        break;
-        NC_LW_CASES(NC_B_CRT_TC32)
-#undef NC_B_CRT_TC32
-        default: break;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(taddr) : "memory");
+    const ProductDesc d = a.products[w.x].d;
+    crt32_cta<LOG_N1>(d, a.tables, int(w.y), crt32_batch_log_tile(int(d.logN)), cols);
 #endif
 }
 
@@ -721,12 +829,26 @@ void* dec_tc32_kernel(int logN1) {
     }
 }
 
-void* crt_tc32_kernel(int LW) {
-    switch (LW) {
-#define NC_CRT_TC32(n) \
-    case n: return reinterpret_cast<void*>(&k_crt_tc32<n>);
-        NC_LW_CASES(NC_CRT_TC32)
-#undef NC_CRT_TC32
+void* crt_tc32_kernel(int logN1) {
+    switch (logN1) {
+        case 0: return reinterpret_cast<void*>(&k_crt_tc32<0>);
+        case 1: return reinterpret_cast<void*>(&k_crt_tc32<1>);
+        case 2: return reinterpret_cast<void*>(&k_crt_tc32<2>);
+        case 3: return reinterpret_cast<void*>(&k_crt_tc32<3>);
+        case 4: return reinterpret_cast<void*>(&k_crt_tc32<4>);
+        case 5: return reinterpret_cast<void*>(&k_crt_tc32<5>);
+        default: return nullptr;
+    }
+}
+
+void* batch_crt_tc32_kernel(int logN1) {
+    switch (logN1) {
+        case 0: return reinterpret_cast<void*>(&k_batch_crt_tc32<0>);
+        case 1: return reinterpret_cast<void*>(&k_batch_crt_tc32<1>);
+        case 2: return reinterpret_cast<void*>(&k_batch_crt_tc32<2>);
+        case 3: return reinterpret_cast<void*>(&k_batch_crt_tc32<3>);
+        case 4: return reinterpret_cast<void*>(&k_batch_crt_tc32<4>);
+        case 5: return reinterpret_cast<void*>(&k_batch_crt_tc32<5>);
         default: return nullptr;
     }
 }
@@ -768,18 +890,18 @@ cudaError_t prepare_w32() {
     for (int l = 0; l <= kMaxLogN1 && e == cudaSuccess; ++l)
         e = cudaFuncSetAttribute(w32::dec_tc32_kernel(l), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(dec_tc32_smem_bytes(kMaxPrimes32)));
-    for (int lw = 2; lw <= kMaxL && e == cudaSuccess; lw += 2)
-        e = cudaFuncSetAttribute(w32::crt_tc32_kernel(lw), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(w32::crt_tc32_smem_bytes(lw)));
+    for (int l = 0; l <= kMaxLogN1 && e == cudaSuccess; ++l)
+        e = cudaFuncSetAttribute(w32::crt_tc32_kernel(l), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(w32::crt_tc32_smem_bytes(kMaxL)));
     for (int l = 0; l <= kMaxLogN1 && e == cudaSuccess; ++l)
         e = cudaFuncSetAttribute(w32::batch_dec_tc32_kernel(l), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(dec_tc32_smem_bytes(kMaxPrimes32)));
     for (int n = 1; n <= kBatchRowLogMax && e == cudaSuccess; ++n)
         e = cudaFuncSetAttribute(w32::persistent_rows32_kernel(n), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(w32::row_smem_bytes(kThreads, kBatchRowLogE)));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(w32::k_batch_crt_tc32, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(w32::crt_tc32_smem_bytes(30)));
+    for (int l = 0; l <= kMaxLogN1 && e == cudaSuccess; ++l)
+        e = cudaFuncSetAttribute(w32::batch_crt_tc32_kernel(l), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(w32::crt_tc32_smem_bytes(kMaxL)));
     return e;
 }
 
@@ -806,11 +928,13 @@ cudaError_t persistent_rows32_occupancy(int logN2, int* ctas_per_sm) {
                                                          w32::row_smem_bytes(kThreads, kBatchRowLogE));
 }
 
-cudaError_t launch_batch_crt_tc32(const BatchCrtArgs& args, int lw_max, cudaStream_t s) {
+cudaError_t launch_batch_crt_tc32(const BatchCrtArgs& args, int logN1, int lw_max, cudaStream_t s) {
+    void* fn = w32::batch_crt_tc32_kernel(logN1);
+    if (!fn) return cudaErrorInvalidValue;
     BatchCrtArgs a = args;
-    void* params[] = {&a};
-    return launch_pdl(reinterpret_cast<void*>(&w32::k_batch_crt_tc32), args.n_items, kThreads,
-                      w32::crt_tc32_smem_bytes(lw_max), s, params);
+    uint32_t cols = crt32_tmem_cols(lw_max);
+    void* params[] = {&a, &cols};
+    return launch_pdl(fn, args.n_items, kThreads, w32::crt_tc32_smem_bytes(lw_max), s, params);
 }
 
 cudaError_t launch_residues32(const ProductDesc& d, const Tables& t, int logN1, cudaStream_t s, int first, int count,
@@ -833,13 +957,16 @@ cudaError_t launch_row32(const ProductDesc& d, const Tables& t, const RowConfig&
     return launch_pdl(fn, g.row_ctas, cfg.threads, w32::row_smem_bytes(cfg.threads, cfg.logE), s, args);
 }
 
-cudaError_t launch_crt32(const ProductDesc& d, const Tables& t, int tiles, cudaStream_t s) {
-    void* fn = w32::crt_tc32_kernel(int(d.LW));
+cudaError_t launch_crt32(const ProductDesc& d, const Tables& t, cudaStream_t s) {
+    const int logN1 = int(d.logN) - int(d.logN2);
+    void* fn = w32::crt_tc32_kernel(logN1);
     if (!fn || !d.crt_b || !d.qc32) return cudaErrorInvalidValue;
     ProductDesc dd = d;
     Tables tt = t;
-    void* args[] = {&dd, &tt};
-    return launch_pdl(fn, tiles, kThreads, w32::crt_tc32_smem_bytes(int(d.LW)), s, args);
+    int logT = crt32_log_tile(int(d.logN), logN1);
+    uint32_t cols = crt32_tmem_cols(int(d.LW));
+    void* args[] = {&dd, &tt, &logT, &cols};
+    return launch_pdl(fn, 1 << (int(d.logN) - logT), kThreads, w32::crt_tc32_smem_bytes(int(d.LW)), s, args);
 }
 
 }  // namespace nc

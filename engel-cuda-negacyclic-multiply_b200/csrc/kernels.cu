@@ -124,7 +124,7 @@ cudaError_t launch_product(const ProductDesc& d, const Tables& t, const RowConfi
     if (ev && (e = cudaEventRecord(ev[2], s)) != cudaSuccess) return e;
     if (d.mode != kModeForward) {
         if (w32) {
-            e = launch_crt32(d, t, g.tiles, s);
+            e = launch_crt32(d, t, s);
         } else {
             void* args[] = {&dd, &tt};
             e = launch(crt, g.tiles, kThreads, d.crt_b ? crt_tc_smem_bytes(int(d.LW)) : crt_smem_bytes(int(d.k)), s,

@@ -71,6 +71,22 @@ __device__ __forceinline__ int swz(int x) {
 // ------------------------------------------------------------------------------------------
 // column stages (registers), as column_forward / column_inverse of the 62-bit engine
 
+// Twiddles (root << s) + blk and the next one: neighbours from stage 1 on, one 16-byte load.
+struct ColumnTwiddles {
+    uint2 w[2];
+};
+__device__ __forceinline__ ColumnTwiddles column_twiddles(const uint2* tw, int at, int s) {
+    ColumnTwiddles r;
+    if (s == 0) {
+        r.w[0] = r.w[1] = __ldg(tw + at);
+    } else {
+        const uint4 pr = __ldg(reinterpret_cast<const uint4*>(tw + at));
+        r.w[0] = make_uint2(pr.x, pr.y);
+        r.w[1] = make_uint2(pr.z, pr.w);
+    }
+    return r;
+}
+
 template <int LOG_N1>
 __device__ __forceinline__ void column_forward_root(const uint2* tw, int root, uint32_t p, uint32_t (&v)[1 << LOG_N1]) {
     constexpr int N1 = 1 << LOG_N1;
@@ -79,12 +95,15 @@ __device__ __forceinline__ void column_forward_root(const uint2* tw, int root, u
     for (int s = 0; s < LOG_N1; ++s) {
         const int half = N1 >> (s + 1);
 #pragma unroll
-        for (int blk = 0; blk < (1 << s); ++blk) {
-            const uint2 w = __ldg(tw + (root << s) + blk);
+        for (int blk = 0; blk < (1 << s); blk += 2) {
+            const ColumnTwiddles w = column_twiddles(tw, (root << s) + blk, s);
 #pragma unroll
-            for (int jj = 0; jj < half; ++jj) {
-                const int u = blk * 2 * half + jj;
-                ct_bfly(v[u], v[u + half], w.x, w.y, p, p2);
+            for (int e = 0; e < (s == 0 ? 1 : 2); ++e) {
+#pragma unroll
+                for (int jj = 0; jj < half; ++jj) {
+                    const int u = (blk + e) * 2 * half + jj;
+                    ct_bfly(v[u], v[u + half], w.w[e].x, w.w[e].y, p, p2);
+                }
             }
         }
     }
@@ -98,12 +117,15 @@ __device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, u
     for (int s = LOG_N1 - 1; s >= 0; --s) {
         const int half = N1 >> (s + 1);
 #pragma unroll
-        for (int blk = 0; blk < (1 << s); ++blk) {
-            const uint2 w = __ldg(tw + (root << s) + blk);
+        for (int blk = 0; blk < (1 << s); blk += 2) {
+            const ColumnTwiddles w = column_twiddles(tw, (root << s) + blk, s);
 #pragma unroll
-            for (int jj = 0; jj < half; ++jj) {
-                const int u = blk * 2 * half + jj;
-                gs_bfly(v[u], v[u + half], w.x, w.y, p, p2);
+            for (int e = 0; e < (s == 0 ? 1 : 2); ++e) {
+#pragma unroll
+                for (int jj = 0; jj < half; ++jj) {
+                    const int u = (blk + e) * 2 * half + jj;
+                    gs_bfly(v[u], v[u + half], w.w[e].x, w.w[e].y, p, p2);
+                }
             }
         }
     }
