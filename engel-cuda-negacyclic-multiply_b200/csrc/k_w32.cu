@@ -5,8 +5,8 @@
 // Residues. With x_n given as 4 L bytes x_{n,b}, x_n mod p_i = sum_c 2^(8 c) S[n][i,c] with
 // S[n][i,c] = sum_b x_{n,b} w_{i,b,c}, w_{i,b,c} byte c (of 4) of 2^(8 b) mod p_i: the same u8 x u8
 // contraction as the 62-bit engine's k_dec_tc, with four byte planes a prime instead of eight, so
-// one pass of MMAs (128 accumulator columns) covers 32 primes. The folded sum (< 2^48) is reduced
-// with one multiply by floor(2^50 / p).
+// one pass of MMAs (128 accumulator columns) covers 32 primes. The four sums are folded and reduced
+// together (fold_planes).
 //
 // CRT. The 4 bytes of each residue against a per-plan table (K = 4 k <= 256 bytes) that carries the
 // factors y_i, the reduction of M/p_i mod q and the quotient (below, at the CRT's kernels).
@@ -42,17 +42,18 @@ __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c)
     return d;
 }
 
-// sum_c 2^(8 c) s[c] mod p into [0, 2p), for s[c] < 2^23 (so the sum V < 2^48) and p in
-// (2^29, 2^30): with A = V >> 28 and bar = floor(2^50 / p), floor(A bar / 2^22) falls short of
-// V / p by less than 2^28 / p + 2^20 / 2^22 < 0.75, so it is floor(V / p) or one less.
-__device__ __forceinline__ uint32_t fold_planes(const uint32_t* s, uint32_t p, uint32_t bar) {
-    const uint64_t v = mad_wide(s[3], 1u << 24, mad_wide(s[2], 1u << 16, mad_wide(s[1], 1u << 8, uint64_t(s[0]))));
-    const uint32_t qh = uint32_t((uint64_t(uint32_t(v >> 28)) * bar) >> 22);
-    return uint32_t(v) - qh * p;
+// sum_c 2^(8 c) s[c] mod p into [0, 3.3 p) (the butterflies take [0, 4p)), for s[c] < 2^23 and p in
+// (2^29.8, 2^30): with lo = s0 + 2^8 s1 and hi = s2 + 2^8 s3 (both below 2^31.01), V = lo + 2^16 hi and
+// q = floor(hi floor(2^48 / p) / 2^32) falls short of 2^16 hi / p by less than 1 + hi / 2^32 < 1.6, and
+// lo < 2.3 p is not reduced: V - q p < 3.9 p. Five instructions, one of them a multiply-high (a 48-bit
+// sum and its Barrett quotient took ten).
+__device__ __forceinline__ uint32_t fold_planes(const uint32_t* s, uint32_t p, uint32_t c48) {
+    const uint32_t lo = s[0] + (s[1] << 8), hi = s[2] + (s[3] << 8);
+    return lo + (hi << 16) - __umulhi(hi, c48) * p;
 }
 
-// Residue row of prime i (128 u32) over its pair's 1 KB of weights.
-__device__ __forceinline__ uint32_t* res_row(uint8_t* sB, int i) { return reinterpret_cast<uint32_t*>(sB + i * 512); }
+// Residue row of prime il of the pass group (128 u32) over its pair's 1 KB of weights.
+__device__ __forceinline__ uint32_t* res_row(uint8_t* sB, int il) { return reinterpret_cast<uint32_t*>(sB + il * 512); }
 
 // Slot of tile row x in prime i's residue row. Every prime's row starts on bank 0, so rows are
 // XORed (bits 2-4 for 4-column tiles, bits 0-4 otherwise) by the prime and, for 4-column tiles,
@@ -67,25 +68,96 @@ __device__ __forceinline__ int res_slot(int i, int x, int C) {
 // multiple of 16 columns), within the table's 64 primes.
 __host__ __device__ constexpr int dec32_weight_pairs(int k) { return ((k + 3) & ~3) / 2; }
 
-// CC: the tile's columns when N >= 128 (128 >> LOG_N1, a constant: the index arithmetic of the
-// fold and the column stages folds away), 0 for smaller N.
-template <int LOG_N1, int CC>
-__device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables& t, int operand, int tile,
-                                              uint8_t* smem, uint64_t& bar, uint32_t& taddr_slot) {
+// Forward column stages of one prime: 2^LOG_N1 points of each of the tile's columns.
+template <int LOG_N1, int CC, int LN2>
+__device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, const uint2* s_pc, uint8_t* sB, int N,
+                                              int N2, int logC, int j0, int i0, int i1) {
     constexpr int N1 = 1 << LOG_N1;
+    const int C = CC ? CC : 1 << logC;
+    const int tid = int(threadIdx.x), lane = tid & 31;
+    if constexpr (LOG_N1 == 5) {
+        // 32-point columns on two adjacent lanes, as in k_dec_tc: lane h runs the first stage's
+        // butterflies (u, u + 16) for u in [8h, 8h + 8), the lanes swap halves, and each runs the
+        // four remaining stages on its half-subtree (twiddle root 2 + h)
+        const int total = 2 * (i1 - i0) * C;
+        for (int w0 = tid & ~31; w0 < total; w0 += kThreads) {
+            const int w = w0 + lane;
+            const bool active = w < total;
+            const int item = active ? w >> 1 : 0, h = w & 1;
+            const int i = i0 + (item >> logC), j = item & (C - 1);
+            const uint32_t* sr = res_row(sB, i - i0);
+            const uint32_t p = s_pc[i - i0].x, p2 = 2 * p;
+            const uint2* tw = tw0 + size_t(i) * kMaxN;
+            uint32_t xs[8], ys[8];
+            const uint2 w1 = __ldg(tw + 1);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const int u = 8 * h + e;
+                xs[e] = sr[res_slot(i, u * C + j, C)];
+                ys[e] = sr[res_slot(i, (u + 16) * C + j, C)];
+                w32::ct_bfly(xs[e], ys[e], w1.x, w1.y, p, p2);
+            }
+            uint32_t v[16];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? xs[e] : ys[e], 1);
+                v[e] = h ? got : xs[e];
+                v[8 + e] = h ? ys[e] : got;
+            }
+            w32::column_forward_root<4>(tw, 2 + h, p, v);
+            if (active) {
+                uint32_t* out = R + size_t(i) * N + j0 + j + size_t(16 * h) * N2;
+#pragma unroll
+                for (int u = 0; u < 16; ++u) __stcg(out + size_t(u) * N2, v[u]);
+            }
+        }
+    } else {
+        const int total = (i1 - i0) << logC;
+#pragma unroll 1
+        for (int w = tid; w < total; w += kThreads) {
+            const int i = i0 + (w >> logC), j = w & (C - 1);
+            const uint32_t* sr = res_row(sB, i - i0);
+            uint32_t v[N1];
+            if constexpr (CC == 8 || CC == 16) {
+                // rows u C + j XORed by (i C) mod 32 are (u ^ (i mod 32 / C)) C + j
+                constexpr int G = 32 / CC;
+                const int e = i & (G - 1);
+                const uint32_t* at[G];
+#pragma unroll
+                for (int b = 0; b < G; ++b) at[b] = sr + ((b ^ e) * CC + j);
+#pragma unroll
+                for (int u = 0; u < N1; ++u) v[u] = at[u & (G - 1)][(u & ~(G - 1)) * CC];
+            } else {
+#pragma unroll
+                for (int u = 0; u < N1; ++u) v[u] = sr[res_slot(i, u * C + j, C)];
+            }
+            if (LOG_N1 > 0) w32::column_forward_root<LOG_N1>(tw0 + size_t(i) * kMaxN, 1, s_pc[i - i0].x, v);
+            uint32_t* out = R + size_t(i) * N + j0 + j;
+#pragma unroll
+            for (int u = 0; u < N1; ++u) __stcg(out + size_t(u) * N2, v[u]);
+        }
+    }
+}
+
+// CC: the tile's columns when N >= 128 (128 >> LOG_N1, a constant: the index arithmetic of the
+// fold and the column stages folds away), 0 for smaller N. LN2: log2 N2 where it is 12 (the stores'
+// offsets are then constants), else 0. Primes [i0, i1), i0 a multiple of 32.
+template <int LOG_N1, int CC, int LN2>
+__device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables& t, int operand, int tile, int i0,
+                                              int i1, uint8_t* smem, uint64_t& bar, uint32_t& taddr_slot) {
     const int N = 1 << d.logN;
-    const int N2 = N >> LOG_N1;
+    const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
     const int T = CC ? kDecTcRows : (N < kDecTcRows ? N : kDecTcRows);
     const int logC = CC ? 7 - LOG_N1 : (N < kDecTcRows ? int(d.logN) : 7) - LOG_N1;
     const int C = CC ? CC : 1 << logC;
     const int j0 = tile * C;
-    const int L = int(d.L), k = int(d.k);
+    const int L = int(d.L), k = i1 - i0;
     const int wpairs = dec32_weight_pairs(k);
     const uint32_t* x = factor_limbs(d, operand);
     uint32_t* R = reinterpret_cast<uint32_t*>(factor_residues(d, operand));
     uint8_t* sA = smem;                     // [16 row groups][8 K chunks][8 rows][16 B]
     uint8_t* sB = smem + kDecTcRows * 128;  // [prime pair][8 K chunks][8 rows][16 B]
-    PrimeConst32* s_pc = reinterpret_cast<PrimeConst32*>(sB + wpairs * 1024);
+    uint2* s_pc = reinterpret_cast<uint2*>(sB + wpairs * 1024);  // p, floor(2^48 / p)
     const int tid = int(threadIdx.x), warp = tid >> 5, lane = tid & 31;
 
     if (warp == 0) {
@@ -98,13 +170,20 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // dependents are released only once every CTA holds its tensor memory (as in k_dec_tc)
     __syncthreads();
-    pdl_trigger();
 
-    for (int q = tid; q < wpairs * 64; q += kThreads) cp_async16(sB + q * 16, t.res_w32 + q);
-    for (int w = tid; w < ((k + 3) & ~3); w += kThreads) s_pc[w] = t.pc32[w];  // the MMAs' primes
+    const uint4* w_src = t.res_w32 + size_t(i0 >> 1) * 64;
+    for (int q = tid; q < wpairs * 64; q += kThreads) cp_async16(sB + q * 16, w_src + q);
+    for (int w = tid; w < 2 * wpairs; w += kThreads) {
+        const PrimeConst32 pc = t.pc32[i0 + w];  // the MMAs' primes
+        s_pc[w] = make_uint2(pc.p, pc.bar >> 2);
+    }
     pdl_wait();  // the operand and the residue rows belong to the stream's previous kernels
+    // after the wait (and with the CTA's tensor memory in hand): the next kernel's CTAs are then placed
+    // beside running CTAs, not beside a queue of waiting ones; at the kernel's entry, products of
+    // N = 4096 to 16384 had kernels of two products resident at once, several row CTAs stacked on one
+    // SM (N = 8192, 868 bits: 28.7 us a product, 20.3 us with the trigger here)
+    pdl_trigger();
     const int kbytes = 4 * L;
     for (int q = tid; q < kDecTcRows * 8; q += kThreads) {
         const int rlo = q & 7, kc = (q >> 3) & 7, rg = q >> 6;
@@ -140,14 +219,18 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     // pass's primes (16 of them, four per 16-column load)
     const int m = 32 * (warp & 3) + lane;
     const int half = warp >> 2;
+    // a prime's place in its residue row depends on the prime mod 4 only (CC a constant)
+    int slot[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) slot[e] = CC ? res_slot(e, m, CC) : 0;
     bool failed = false;
     for (int g = 0; g * kDecTc32PassPrimes < k; ++g) {
-        const int i0 = g * kDecTc32PassPrimes;
-        const int np = k - i0 < kDecTc32PassPrimes ? k - i0 : kDecTc32PassPrimes;
+        const int ig = g * kDecTc32PassPrimes;
+        const int np = k - ig < kDecTc32PassPrimes ? k - ig : kDecTc32PassPrimes;
         if (tid == 0 && !failed) {
             const uint32_t ncols = uint32_t(((np + 3) & ~3) * 4);
             const uint32_t idesc = (2u << 4) | ((ncols >> 3) << 17) | (uint32_t(kDecTcRows >> 4) << 24);
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB + (i0 >> 1) * 1024);
+            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB + (ig >> 1) * 1024);
             for (int s = 0; s < slices; ++s) {
                 const uint64_t da = kmajor_desc(a0 + uint32_t(s) * 256u, 128u, 1024u);
                 const uint64_t db = kmajor_desc(b0 + uint32_t(s) * 256u, 128u, 1024u);
@@ -163,10 +246,11 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
         }
         const bool ok = !failed && mma_wait(smem_u32(&bar), uint32_t(g & 1));
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int ib = i0 + 16 * half;
-        const int ie = i0 + np < ib + 16 ? i0 + np : ib + 16;
+        const int ib = ig + 16 * half;
+        const int ie = ig + np < ib + 16 ? ig + np : ib + 16;
         if (__all_sync(0xffffffffu, ok)) {
             const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16);
+#pragma unroll 1
             for (int i = ib; i < ie; i += 4) {
                 uint32_t s[16];
                 asm volatile(
@@ -175,23 +259,26 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
                     : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]),
                       "=r"(s[8]), "=r"(s[9]), "=r"(s[10]), "=r"(s[11]), "=r"(s[12]), "=r"(s[13]), "=r"(s[14]),
                       "=r"(s[15])
-                    : "r"(lane_base + uint32_t(4 * (i - i0))));
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    : "r"(lane_base + uint32_t(4 * (i - ig))));
                 // all four (primes up to k rounded up to four have weights, constants and rows)
+                const uint4 c01 = *reinterpret_cast<const uint4*>(s_pc + i), c23 = *reinterpret_cast<const uint4*>(s_pc + i + 2);
+                const uint32_t p[4] = {c01.x, c01.z, c23.x, c23.z}, c48[4] = {c01.y, c01.w, c23.y, c23.w};
+                uint32_t* rows = res_row(sB, i);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
-                    res_row(sB, i + e)[res_slot(i + e, m, C)] = fold_planes(s + 4 * e, s_pc[i + e].p, s_pc[i + e].bar);
+                    rows[128 * e + (CC ? slot[e] : res_slot(i0 + i + e, m, C))] = fold_planes(s + 4 * e, p[e], c48[e]);
             }
         } else if (m < T) {
             // the wait gave up: this warp's residues on the integer pipes
             const int n = (m >> logC) * N2 + j0 + (m & (C - 1));
             const uint32_t* row = x + size_t(n) * size_t(L);
             for (int i = ib; i < ie; ++i) {
-                const uint64_t p = s_pc[i].p;
+                const uint64_t p = s_pc[i].x;
                 uint64_t acc = 0;
                 for (int l = 0; l < L; ++l)
-                    acc = (acc + uint64_t(__ldg(row + l)) * __ldg(t.pow32_32 + size_t(i) * kMaxL + l)) % p;
-                res_row(sB, i)[res_slot(i, m, C)] = uint32_t(acc);
+                    acc = (acc + uint64_t(__ldg(row + l)) * __ldg(t.pow32_32 + size_t(i0 + i) * kMaxL + l)) % p;
+                res_row(sB, i)[res_slot(i0 + i, m, C)] = uint32_t(acc);
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -200,72 +287,39 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kDecTcCols) : "memory");
-
-    // forward column stages of items (prime i, column j), then the residue rows
-    if constexpr (LOG_N1 == 5) {
-        // 32-point columns on two adjacent lanes, as in k_dec_tc: lane h runs the first stage's
-        // butterflies (u, u + 16) for u in [8h, 8h + 8), the lanes swap halves, and each runs the
-        // four remaining stages on its half-subtree (twiddle root 2 + h)
-        const int total = 2 * k * C;
-        for (int w0 = tid & ~31; w0 < total; w0 += kThreads) {
-            const int w = w0 + lane;
-            const bool active = w < total;
-            const int item = active ? w >> 1 : 0, h = w & 1;
-            const int i = item >> logC, j = item & (C - 1);
-            const uint32_t* sr = res_row(sB, i);
-            const uint32_t p = s_pc[i].p, p2 = 2 * p;
-            const uint2* tw = t.fwd32 + size_t(i) * kMaxN;
-            uint32_t xs[8], ys[8];
-            const uint2 w1 = __ldg(tw + 1);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int u = 8 * h + e;
-                xs[e] = sr[res_slot(i, u * C + j, C)];
-                ys[e] = sr[res_slot(i, (u + 16) * C + j, C)];
-                w32::ct_bfly(xs[e], ys[e], w1.x, w1.y, p, p2);
-            }
-            uint32_t v[16];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? xs[e] : ys[e], 1);
-                v[e] = h ? got : xs[e];
-                v[8 + e] = h ? ys[e] : got;
-            }
-            w32::column_forward_root<4>(tw, 2 + h, p, v);
-            if (active) {
-                uint32_t* out = R + size_t(i) * N + j0 + j + size_t(16 * h) * N2;
-#pragma unroll
-                for (int u = 0; u < 16; ++u) __stcg(out + size_t(u) * N2, v[u]);
-            }
-        }
-    } else {
-        for (int w = tid; w < k * C; w += kThreads) {
-            const int i = w >> logC, j = w & (C - 1);
-            const uint32_t* sr = res_row(sB, i);
-            uint32_t v[N1];
-#pragma unroll
-            for (int u = 0; u < N1; ++u) v[u] = sr[res_slot(i, u * C + j, C)];
-            if (LOG_N1 > 0) w32::column_forward_root<LOG_N1>(t.fwd32 + size_t(i) * kMaxN, 1, s_pc[i].p, v);
-            uint32_t* out = R + size_t(i) * N + j0 + j;
-#pragma unroll
-            for (int u = 0; u < N1; ++u) __stcg(out + size_t(u) * N2, v[u]);
-        }
-    }
+    dec32_columns<LOG_N1, CC, LN2>(R, t.fwd32, s_pc, sB, N, N2, logC, j0, i0, i1);
 }
 
-// Four CTAs per SM, as k_dec_tc (tensor memory holds four of 128 columns).
+// The item by its tile width and row length.
+template <int LOG_N1>
+__device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables& t, int operand, int tile, int i0, int i1,
+                                             uint8_t* smem, uint64_t& bar, uint32_t& taddr_slot) {
+    if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
+        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 12>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+    else if (d.logN >= 7)
+        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 0>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+    else
+        dec_tc32_item<LOG_N1, 0, 0>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+}
+
+// Four CTAs per SM, as k_dec_tc (tensor memory holds four of 128 columns). With `split`, a CTA takes
+// one pass of 32 primes of its tile instead of all of them (small grids: every pass is then a CTA
+// of its own).
 template <int LOG_N1>
 __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables t, int first_operand, int tile0,
-                                                           int tiles) {
+                                                           int tiles, int split) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bar;
     __shared__ uint32_t taddr_slot;
-    const int operand = first_operand + int(blockIdx.x) / tiles, tile = tile0 + int(blockIdx.x) % tiles;
-    if (d.logN >= 7)
-        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1)>(d, t, operand, tile, smem, bar, taddr_slot);
-    else
-        dec_tc32_item<LOG_N1, 0>(d, t, operand, tile, smem, bar, taddr_slot);
+    int b = int(blockIdx.x), i0 = 0, i1 = int(d.k);
+    if (split) {
+        const int passes = (i1 + kDecTc32PassPrimes - 1) / kDecTc32PassPrimes;
+        i0 = (b % passes) * kDecTc32PassPrimes;
+        if (i1 > i0 + kDecTc32PassPrimes) i1 = i0 + kDecTc32PassPrimes;
+        b /= passes;
+    }
+    dec_tc32_any<LOG_N1>(d, t, first_operand + b / tiles, tile0 + b % tiles, i0, i1, smem, bar, taddr_slot);
 #endif
 }
 
@@ -687,10 +741,9 @@ template <int LOG_N2, int LOG_E, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3) : 2)) k_row32(ProductDesc d, Tables t) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bar;
-    pdl_trigger();
     const uint32_t b = smem_u32(&bar);
     w32::row_barrier_init<LOG_N2, LOG_E, THREADS>(b);
-    w32::row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem, b, 0, true);
+    w32::row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem, b, 0, true, true);
 }
 
 #define NC_ROW32_VARIANTS(X)                                                                                   \
@@ -715,10 +768,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_dec_tc32(BatchCrtArgs a) 
     const BatchProduct& bp = a.products[w.x];
     const int tiles = int(bp.tiles_tc);
     const int operand = int(bp.first_operand) + int(w.y) / tiles, tile = int(w.y) % tiles;
-    if (bp.d.logN >= 7)
-        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1)>(bp.d, a.tables, operand, tile, smem, bar, taddr_slot);
-    else
-        dec_tc32_item<LOG_N1, 0>(bp.d, a.tables, operand, tile, smem, bar, taddr_slot);
+    dec_tc32_any<LOG_N1>(bp.d, a.tables, operand, tile, 0, int(bp.d.k), smem, bar, taddr_slot);
 #endif
 }
 
@@ -857,6 +907,9 @@ void* batch_crt_tc32_kernel(int logN1) {
 
 }  // namespace w32
 
+// Residue launches of at most this many CTAs give each pass of primes its own CTA.
+constexpr int kDec32SplitCtas = 74;
+
 // Shared memory of the 30-bit residue stage: the limb tile, the weights of the primes it
 // copies and their constants; raised, as dec_tc_smem_bytes, to keep four CTAs per SM.
 size_t dec_tc32_smem_bytes(int k) {
@@ -943,8 +996,14 @@ cudaError_t launch_residues32(const ProductDesc& d, const Tables& t, int logN1, 
     if (!fn || !t.res_w32 || int(d.k) > kMaxPrimes32) return cudaErrorInvalidValue;
     ProductDesc dd = d;
     Tables tt = t;
-    void* args[] = {&dd, &tt, &first, &tile0, &tiles};
-    return launch_pdl(fn, count * tiles, kThreads, dec_tc32_smem_bytes(int(d.k)), s, args);
+    // a pass of 32 primes a CTA while that leaves half the SMs free: the passes of a tile then run
+    // side by side (868 bits, N = 1024: 16.4 -> 15.3 us a product; N = 4096, 128 CTAs and a short
+    // second pass at 600 bits: 18.2 -> 22.6 us, so not there)
+    const int passes = (int(d.k) + kDecTc32PassPrimes - 1) / kDecTc32PassPrimes;
+    int split = count * tiles * passes <= kDec32SplitCtas ? 1 : 0;
+    const int primes = split && int(d.k) > kDecTc32PassPrimes ? kDecTc32PassPrimes : int(d.k);
+    void* args[] = {&dd, &tt, &first, &tile0, &tiles, &split};
+    return launch_pdl(fn, count * tiles * (split ? passes : 1), kThreads, dec_tc32_smem_bytes(primes), s, args);
 }
 
 cudaError_t launch_row32(const ProductDesc& d, const Tables& t, const RowConfig& cfg, cudaStream_t s) {

@@ -330,7 +330,8 @@ __device__ __forceinline__ void copy_twiddles(const uint2* tw, int base, uint2* 
 // CTA's mbarrier `bar` (row_barrier_init), phase `parity` (a persistent CTA's items alternate
 // phases): the passes then wait on no global load. use_bulk false (a persistent CTA after a bulk
 // wait gave up) loads them with plain loads instead. Returns false if this item's bulk wait gave
-// up (its data then came by plain loads, so the item's result stands).
+// up (its data then came by plain loads, so the item's result stands). With `trigger`, the next kernel
+// may be scheduled once the residues are there (a kernel of one item a CTA).
 template <int LOG_N2, int LOG_E, int THREADS>
 __device__ __forceinline__ void row_barrier_init(uint32_t bar) {
     using S = RowShape<LOG_N2, LOG_E>;
@@ -347,7 +348,7 @@ __device__ __forceinline__ void row_barrier_init(uint32_t bar) {
 
 template <int LOG_N2, int LOG_E, int THREADS>
 __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t, int item, uint8_t* smem,
-                                           uint32_t bar, uint32_t parity, bool use_bulk) {
+                                           uint32_t bar, uint32_t parity, bool use_bulk, bool trigger = false) {
     using S = RowShape<LOG_N2, LOG_E>;
     static_assert(S::T <= THREADS, "row block needs more threads than the CTA has");
     constexpr int ROWS = THREADS / S::T;
@@ -403,6 +404,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
     };
 
     pdl_wait();  // the residues come from the stream's previous kernel
+    if (trigger) pdl_trigger();
     // the residue blocks as bulk copies too (16-byte aligned for blocks of 4 and more): product
     // and forward modes put a's block in buf_a and (with PF_B) b's in b_in; cached-a mode a_hat's
     // block in buf and b's in buf_a. They are read in the first pass's layout, before any thread
