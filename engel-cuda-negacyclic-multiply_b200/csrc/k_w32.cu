@@ -68,6 +68,11 @@ __device__ __forceinline__ int res_slot(int i, int x, int C) {
 // multiple of 16 columns), within the table's 64 primes.
 __host__ __device__ constexpr int dec32_weight_pairs(int k) { return ((k + 3) & ~3) / 2; }
 
+// Neighbouring columns a thread of the column stages takes (VJ): sixteen values in registers. Thirty-two
+// spill at 64 registers and leave threads idle (64 x 16384, 8-point columns: 946, 897 and 983 us a batch
+// with one, two and four columns; N = 65536, 16-point columns: 74.9 and 76.1 us a product with one and two).
+__host__ __device__ constexpr int column_width(int logN1) { return logN1 <= 2 ? 4 : logN1 == 3 ? 2 : 1; }
+
 // Forward column stages of one prime: 2^LOG_N1 points of each of the tile's columns.
 template <int LOG_N1, int CC, int LN2>
 __device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, const uint2* s_pc, uint8_t* sB, int N,
@@ -97,18 +102,61 @@ __device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, con
                 ys[e] = sr[res_slot(i, (u + 16) * C + j, C)];
                 w32::ct_bfly(xs[e], ys[e], w1.x, w1.y, p, p2);
             }
-            uint32_t v[16];
+            uint32_t v[1][16];
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
                 const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? xs[e] : ys[e], 1);
-                v[e] = h ? got : xs[e];
-                v[8 + e] = h ? ys[e] : got;
+                v[0][e] = h ? got : xs[e];
+                v[0][8 + e] = h ? ys[e] : got;
             }
-            w32::column_forward_root<4>(tw, 2 + h, p, v);
+            w32::column_forward_root<4, 1>(tw, 2 + h, p, v);
             if (active) {
                 uint32_t* out = R + size_t(i) * N + j0 + j + size_t(16 * h) * N2;
 #pragma unroll
-                for (int u = 0; u < 16; ++u) __stcg(out + size_t(u) * N2, v[u]);
+                for (int u = 0; u < 16; ++u) __stcg(out + size_t(u) * N2, v[0][u]);
+            }
+        }
+    } else if constexpr (CC > 0) {
+        // VJ neighbouring columns of a prime a thread: 16- or 8-byte shared loads and stores, and one set
+        // of twiddles and addresses for all of them. Rows u C + j
+        // XORed by (i C) mod 32 are (u ^ (i mod 32 / C)) C + j.
+        constexpr int VJ = column_width(LOG_N1), GP = CC / VJ;
+        constexpr int X = CC < 32 ? 32 / CC : 1;
+        const int total = (i1 - i0) * GP;
+#pragma unroll 1
+        for (int w = tid; w < total; w += kThreads) {
+            const int il = w / GP, j = (w % GP) * VJ;
+            const int x = il & (X - 1);  // i0 is a multiple of 32
+            const uint32_t* sr = res_row(sB, il) + j;
+            const uint32_t p = s_pc[il].x;
+            uint32_t v[VJ][N1];
+#pragma unroll
+            for (int u = 0; u < N1; ++u) {
+                const uint32_t* at = sr + ((u & ~(X - 1)) + ((u & (X - 1)) ^ x)) * CC;
+                if constexpr (VJ == 4) {
+                    const uint4 q = *reinterpret_cast<const uint4*>(at);
+                    v[0][u] = q.x;
+                    v[1][u] = q.y;
+                    v[2][u] = q.z;
+                    v[3][u] = q.w;
+                } else if constexpr (VJ == 2) {
+                    const uint2 q = *reinterpret_cast<const uint2*>(at);
+                    v[0][u] = q.x;
+                    v[1][u] = q.y;
+                } else {
+                    v[0][u] = *at;
+                }
+            }
+            if (LOG_N1 > 0) w32::column_forward_root<LOG_N1, VJ>(tw0 + size_t(i0 + il) * kMaxN, 1, p, v);
+            uint32_t* out = R + size_t(i0 + il) * N + j0 + j;
+#pragma unroll
+            for (int u = 0; u < N1; ++u) {
+                if constexpr (VJ == 4)
+                    __stcg(reinterpret_cast<uint4*>(out + size_t(u) * N2), make_uint4(v[0][u], v[1][u], v[2][u], v[3][u]));
+                else if constexpr (VJ == 2)
+                    __stcg(reinterpret_cast<uint2*>(out + size_t(u) * N2), make_uint2(v[0][u], v[1][u]));
+                else
+                    __stcg(out + size_t(u) * N2, v[0][u]);
             }
         }
     } else {
@@ -117,24 +165,13 @@ __device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, con
         for (int w = tid; w < total; w += kThreads) {
             const int i = i0 + (w >> logC), j = w & (C - 1);
             const uint32_t* sr = res_row(sB, i - i0);
-            uint32_t v[N1];
-            if constexpr (CC == 8 || CC == 16) {
-                // rows u C + j XORed by (i C) mod 32 are (u ^ (i mod 32 / C)) C + j
-                constexpr int G = 32 / CC;
-                const int e = i & (G - 1);
-                const uint32_t* at[G];
+            uint32_t v[1][N1];
 #pragma unroll
-                for (int b = 0; b < G; ++b) at[b] = sr + ((b ^ e) * CC + j);
-#pragma unroll
-                for (int u = 0; u < N1; ++u) v[u] = at[u & (G - 1)][(u & ~(G - 1)) * CC];
-            } else {
-#pragma unroll
-                for (int u = 0; u < N1; ++u) v[u] = sr[res_slot(i, u * C + j, C)];
-            }
-            if (LOG_N1 > 0) w32::column_forward_root<LOG_N1>(tw0 + size_t(i) * kMaxN, 1, s_pc[i - i0].x, v);
+            for (int u = 0; u < N1; ++u) v[0][u] = sr[res_slot(i, u * C + j, C)];
+            if (LOG_N1 > 0) w32::column_forward_root<LOG_N1, 1>(tw0 + size_t(i) * kMaxN, 1, s_pc[i - i0].x, v);
             uint32_t* out = R + size_t(i) * N + j0 + j;
 #pragma unroll
-            for (int u = 0; u < N1; ++u) __stcg(out + size_t(u) * N2, v[u]);
+            for (int u = 0; u < N1; ++u) __stcg(out + size_t(u) * N2, v[0][u]);
         }
     }
 }
@@ -244,14 +281,17 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
                              smem_u32(&bar))
                          : "memory");
         }
-        const bool ok = !failed && mma_wait(smem_u32(&bar), uint32_t(g & 1));
+        // one warp polls, the others wait at the barrier (eight polling warps took an eighth of the issue slots)
+        const bool ok = __syncthreads_and(warp != 0 || (!failed && mma_wait(smem_u32(&bar), uint32_t(g & 1))) ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int ib = ig + 16 * half;
         const int ie = ig + np < ib + 16 ? ig + np : ib + 16;
-        if (__all_sync(0xffffffffu, ok)) {
+        if (ok) {
             const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16);
-#pragma unroll 1
-            for (int i = ib; i < ie; i += 4) {
+#pragma unroll
+            for (int h4 = 0; h4 < 16; h4 += 4) {
+                const int i = ib + h4;
+                if (i >= ie) break;
                 uint32_t s[16];
                 asm volatile(
                     "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
@@ -282,7 +322,8 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        failed = __syncthreads_or(ok ? 0 : 1) != 0;  // also: this pass's reads are done before the next MMA
+        failed = !ok;
+        __syncthreads();  // this pass's reads are done before the next MMA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (warp == 0)
@@ -337,22 +378,29 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
 //
 // What bounds it: the column butterflies and loads (59 residues of a coefficient against one
 // contraction row), so integer issue and load latency, not the tensor cores. 128-coefficient tiles
-// with the primes in passes of 32 through one 16 KB A buffer keep a CTA at 49 KB, four per SM.
+// with the primes in passes of 32 through one 20 KB A buffer keep a CTA at 54 KB, four per SM.
 
-// Byte offset of (row, prime il of the pass) in A: [16 row groups][8 K chunks][8 rows][16 B].
-__device__ __forceinline__ int crt32_at(int row, int il) {
-    return (row >> 3) * 1024 + (il >> 2) * 128 + (row & 7) * 16 + (il & 3) * 4;
-}
+// A: [16 row groups][8 K chunks of four primes][8 rows][16 B], the chunks 16 or 32 bytes and the row
+// groups 16 bytes further apart than packed: a warp's four-byte stores (eight groups of neighbouring
+// columns x four primes, or four x eight) then fall on 32 banks.
+template <int LOG_N1>
+struct Crt32Layout {
+    static constexpr int kChunk = LOG_N1 == 4 ? 144 : 160;
+    static constexpr int kGroup = 8 * kChunk + 16;
+    __device__ static int at(int row, int il) {
+        return (row >> 3) * kGroup + (il >> 2) * kChunk + (row & 7) * 16 + (il & 3) * 4;
+    }
+};
+constexpr int kCrt32ABytes = 16 * (8 * 160 + 16);
 
 // Primes [i0, i0 + np) of the tile's 2^logC columns: N1 residues at stride N2 (2^LN2, or N / N1 with
-// LN2 0), the inverse stages of the merged tree, four bytes each into A. Items (prime, column) with
-// eight columns of four primes to a warp: its loads are whole sectors and its four-byte stores fall
-// on 32 banks. Both strides are loop constants (rows u C + j with C >= 8 are C * 128 bytes apart in
-// A): 18 multiply-adds a residue went to addresses before. Short columns (N1 <= 4) are loaded
-// several items at a time: one load after another would be the stage's whole time at small N.
-template <int LOG_N1, int LN2>
+// LN2 0), the inverse stages of the merged tree, four bytes each into A. A thread takes VJ neighbouring
+// columns of a prime (16- or 8-byte loads, one set of twiddles and addresses); one-residue loads were most
+// of the stage's instructions at small N1, and their latency its time. Tiles of fewer columns go one by one.
+template <int LOG_N1, int LN2, int VJ>
 __device__ __forceinline__ void crt32_columns(const uint32_t* res, const uint2* tw0, int logN, int logC, int np,
-                                           const uint32_t* s_p, uint8_t* sA) {
+                                              const uint32_t* s_p, uint8_t* sA) {
+    using A = Crt32Layout<LOG_N1>;
     constexpr int N1 = 1 << LOG_N1;
     const int N = 1 << logN;
     const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
@@ -370,65 +418,70 @@ __device__ __forceinline__ void crt32_columns(const uint32_t* res, const uint2* 
             const int item = active ? w >> 1 : 0, h = w & 1;
             const int i = item >> logC, j = item & (C - 1);
             const uint32_t* row = res + size_t(i) * N + j + size_t(16 * h) * N2;
-            uint32_t v[16];
+            uint32_t v[1][16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) v[u] = active ? __ldcg(row + size_t(u) * N2) : 0u;
+            for (int u = 0; u < 16; ++u) v[0][u] = active ? __ldcg(row + size_t(u) * N2) : 0u;
             const uint32_t p = s_p[i], p2 = 2 * p;
             const uint2* tw = tw0 + size_t(i) * kMaxN;
-            w32::column_inverse_root<4>(tw, 2 + h, p, v);
+            w32::column_inverse_root<4, 1>(tw, 2 + h, p, v);
             const uint2 w1 = __ldg(tw + 1);
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? v[e] : v[8 + e], 1);
-                uint32_t lo = h ? got : v[e], hi = h ? v[8 + e] : got;  // rows 8h + e and 8h + e + 16
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, h ? v[0][e] : v[0][8 + e], 1);
+                uint32_t lo = h ? got : v[0][e], hi = h ? v[0][8 + e] : got;  // rows 8h + e and 8h + e + 16
                 w32::gs_bfly(lo, hi, w1.x, w1.y, p, p2);
                 if (active) {
-                    *reinterpret_cast<uint32_t*>(sA + crt32_at((8 * h + e) * C + j, i)) = lo;
-                    *reinterpret_cast<uint32_t*>(sA + crt32_at((8 * h + e + 16) * C + j, i)) = hi;
+                    *reinterpret_cast<uint32_t*>(sA + A::at((8 * h + e) * C + j, i)) = lo;
+                    *reinterpret_cast<uint32_t*>(sA + A::at((8 * h + e + 16) * C + j, i)) = hi;
                 }
             }
         }
     } else {
-        constexpr int U = LOG_N1 >= 3 ? 1 : 8 >> LOG_N1;  // items in flight per thread
-        const bool wide = logC >= 3;
-        const int total = (wide ? (np + 3) & ~3 : np) << logC;
-        auto split = [&](int w, int& i, int& j) {
-            if (wide) {
-                const int hi = w >> 5;
-                i = ((hi >> (logC - 3)) << 2) + ((w >> 3) & 3);
-                j = ((hi & ((C >> 3) - 1)) << 3) + (w & 7);
-            } else {
-                i = w >> logC;
-                j = w & (C - 1);
-            }
-        };
+        constexpr int LV = VJ == 4 ? 2 : VJ == 2 ? 1 : 0;
+        // lanes: up to eight groups of columns (2^logL) of one prime, then primes, then further groups
+        const int logG = logC - LV, logL = logG < 3 ? logG : 3;
+        const int primes = (np + 3) & ~3;
+        const int total = primes << logG;
 #pragma unroll 1
-        for (int w0 = tid; w0 < total; w0 += kThreads * U) {
-            uint32_t v[U][N1];
+        for (int w = tid; w < total; w += kThreads) {
+            const int low = w & ((1 << logL) - 1), mid = w >> logL;
+            // mid walks the primes four at a time within each further run of 2^logL groups
+            const int run = (mid >> 2) & ((1 << (logG - logL)) - 1);
+            const int il = ((mid >> (2 + logG - logL)) << 2) + (mid & 3);
+            const int j = ((run << logL) + low) << LV;
+            if (il >= np) continue;
+            const uint32_t* row = res + size_t(il) * N + j;
+            uint32_t v[VJ][N1];
 #pragma unroll
-            for (int q = 0; q < U; ++q) {
-                int i, j;
-                split(w0 + q * kThreads, i, j);
-                const bool active = w0 + q * kThreads < total && i < np;
-                const uint32_t* row = res + (active ? size_t(i) * N + j : size_t(0));
-#pragma unroll
-                for (int u = 0; u < N1; ++u) v[q][u] = __ldcg(row + size_t(u) * N2);
-            }
-#pragma unroll
-            for (int q = 0; q < U; ++q) {
-                int i, j;
-                split(w0 + q * kThreads, i, j);
-                if (w0 + q * kThreads < total && i < np) {
-                    if (LOG_N1 > 0) w32::column_inverse_root<LOG_N1>(tw0 + size_t(i) * kMaxN, 1, s_p[i], v[q]);
-                    if (wide) {
-                        uint8_t* at = sA + crt32_at(j, i);
-#pragma unroll
-                        for (int u = 0; u < N1; ++u) *reinterpret_cast<uint32_t*>(at + (u << logC) * 128) = v[q][u];
-                    } else {
-#pragma unroll
-                        for (int u = 0; u < N1; ++u) *reinterpret_cast<uint32_t*>(sA + crt32_at(u * C + j, i)) = v[q][u];
-                    }
+            for (int u = 0; u < N1; ++u) {
+                if constexpr (VJ == 4) {
+                    const uint4 q = __ldcg(reinterpret_cast<const uint4*>(row + size_t(u) * N2));
+                    v[0][u] = q.x;
+                    v[1][u] = q.y;
+                    v[2][u] = q.z;
+                    v[3][u] = q.w;
+                } else if constexpr (VJ == 2) {
+                    const uint2 q = __ldcg(reinterpret_cast<const uint2*>(row + size_t(u) * N2));
+                    v[0][u] = q.x;
+                    v[1][u] = q.y;
+                } else {
+                    v[0][u] = __ldcg(row + size_t(u) * N2);
                 }
+            }
+            if (LOG_N1 > 0) w32::column_inverse_root<LOG_N1, VJ>(tw0 + size_t(il) * kMaxN, 1, s_p[il], v);
+            if (logC >= 3) {
+                // rows u C + j are a constant distance apart, and VJ neighbours lie in one row group
+                uint8_t* at = sA + A::at(j, il);
+                const int step = (C >> 3) * A::kGroup;
+#pragma unroll
+                for (int u = 0; u < N1; ++u)
+#pragma unroll
+                    for (int e = 0; e < VJ; ++e) *reinterpret_cast<uint32_t*>(at + u * step + 16 * e) = v[e][u];
+            } else {
+#pragma unroll
+                for (int u = 0; u < N1; ++u)
+#pragma unroll
+                    for (int e = 0; e < VJ; ++e) *reinterpret_cast<uint32_t*>(sA + A::at(u * C + j + e, il)) = v[e][u];
             }
         }
     }
@@ -450,11 +503,11 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 constexpr int kCrt32Words = 36;
 
 // This thread's coefficient from its lane of the accumulator, T mod q, to L limbs at `o` (if `store`).
-// All the lanes of a warp together (tensor-memory loads). Not inlined: one copy for each LW serves the
-// kernels of every column length, and at its call nothing of theirs is live.
+// All the lanes of a warp together (tensor-memory loads).
 template <int LW>
-__device__ __noinline__ void crt32_finish(const QConst32* qc, const uint32_t* s_negm, const uint32_t* s_nq,
-                                          const uint32_t* s_q, uint32_t lane_base, int L, uint32_t* o, bool store) {
+__device__ __forceinline__ void crt32_finish(const QConst32* qc, const uint32_t* s_consts, uint32_t lane_base, int L,
+                                             uint32_t* o, bool store) {
+    const uint32_t *s_negm = s_consts, *s_nq = s_consts + kCrt32Words, *s_q = s_consts + 2 * kCrt32Words;
     uint32_t r[LW + 1];
     const int c0 = int(__ldg(&qc->top_byte)), sh = __ldg(&qc->top_shift);
     uint32_t ph[4], top[8];
@@ -532,7 +585,7 @@ __device__ __noinline__ void crt32_finish(const QConst32* qc, const uint32_t* s_
 // completion in time: the column sum from its definition, x_u N1 = sum_u' z_u' rho_u'^-2u with rho_u'
 // the forward twiddle of row block u' (node N1 + u'), then v_i = r_i y_i and the carry chains.
 template <int LW>
-__device__ __noinline__ void crt32_coeff_plain(const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
+__device__ __forceinline__ void crt32_coeff_plain(const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
                                                const uint2* inv, int logN, int logN1, int k, int L, int u, int j,
                                                uint32_t* out) {
     constexpr int W = LW + kAccExtra;
@@ -573,11 +626,36 @@ __device__ __noinline__ void crt32_coeff_plain(const uint32_t* res, const QConst
     for (int l = 0; l < L; ++l) out[l] = r[l];
 }
 
+// Both by LW, not inlined: one copy serves the kernels of every column length, and at the call next to
+// nothing of theirs is live.
+__device__ __noinline__ void crt32_finish_any(int LW, const QConst32* qc, const uint32_t* s_consts, uint32_t lane_base,
+                                              int L, uint32_t* o, bool store) {
+    switch (LW) {
+#define NC_CRT32_FINISH(n) \
+    case n: crt32_finish<n>(qc, s_consts, lane_base, L, o, store); break;
+        NC_LW_CASES(NC_CRT32_FINISH)
+#undef NC_CRT32_FINISH
+        default: break;
+    }
+}
+
+__device__ __noinline__ void crt32_plain_any(int LW, const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
+                                             const uint2* inv, int logN, int logN1, int k, int L, int u, int j,
+                                             uint32_t* out) {
+    switch (LW) {
+#define NC_CRT32_PLAIN(n) \
+    case n: crt32_coeff_plain<n>(res, qc, pc, inv, logN, logN1, k, L, u, j, out); break;
+        NC_LW_CASES(NC_CRT32_PLAIN)
+#undef NC_CRT32_PLAIN
+        default: break;
+    }
+}
+
 // Shared memory: A (128 rows x the 128 K bytes of 32 primes; the output tile once the sums are
 // out), the finish's constants, p of up to 64 primes, the plan's table; raised so that no more CTAs
 // share an SM than its tensor memory holds.
 NC_HD constexpr size_t crt_tc32_smem_bytes(int LW) {
-    return smax(size_t(kCrt32Rows) * 128 + crt32_table_bytes(LW) + size_t(kMaxPrimes32) * 4 + size_t(kCrt32Words) * 4 * 3,
+    return smax(size_t(kCrt32ABytes) + crt32_table_bytes(LW) + size_t(kMaxPrimes32) * 4 + size_t(kCrt32Words) * 4 * 3,
                 (size_t(233472) / (512 / crt32_tmem_cols(LW) + 1) + 16) / 16 * 16);
 }
 
@@ -603,8 +681,12 @@ __device__ __forceinline__ void crt32_store(uint32_t* c, int N2, int L, int j0, 
 template <int LOG_N1, int LN2>
 __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
                                                 uint8_t* smem, uint32_t taddr, uint64_t* bar) {
-    const int LW = int(d.LW), NC = crt32_cols(LW);
-    const int N = 1 << d.logN;
+    using A = Crt32Layout<LOG_N1>;
+    // the descriptor's fields once (a batch's lies in global memory)
+    const int LW = int(d.LW), NC = crt32_cols(LW), logN = int(d.logN);
+    const uint32_t* ra = reinterpret_cast<const uint32_t*>(d.ra);
+    uint32_t* const c_out = d.c;
+    const int N = 1 << logN;
     const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
     const int T = 1 << logT;
     const int logC = logT - LOG_N1, C = 1 << logC;
@@ -612,7 +694,7 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
     const int j0 = tile * C;
 
     uint8_t* sA = smem;
-    uint32_t* s_negm = reinterpret_cast<uint32_t*>(sA + kCrt32Rows * 128);
+    uint32_t* s_negm = reinterpret_cast<uint32_t*>(sA + kCrt32ABytes);
     uint32_t* s_nq = s_negm + kCrt32Words;
     uint32_t* s_q = s_nq + kCrt32Words;
     uint32_t* s_p = s_q + kCrt32Words;
@@ -642,11 +724,15 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
 #pragma unroll 1
     for (int g = 0; g < passes; ++g) {
         // the A buffer is free once the pass before has been read
-        if (g > 0) ok = __syncthreads_and(ok && mma_wait(bar_addr, uint32_t((g - 1) & 1)) ? 1 : 0) != 0;
+        if (g > 0) ok = __syncthreads_and(warp != 0 || mma_wait(bar_addr, uint32_t((g - 1) & 1)) ? 1 : 0) != 0;
         if (!ok) break;
         const int i0 = 32 * g, np = k - i0 < 32 ? k - i0 : 32;
-        crt32_columns<LOG_N1, LN2>(reinterpret_cast<const uint32_t*>(d.ra) + size_t(i0) * N + j0,
-                                   t.inv32 + size_t(i0) * kMaxN, int(d.logN), logC, np, s_p + i0, sA);
+        const uint32_t* res = ra + size_t(i0) * N + j0;
+        constexpr int VJ = column_width(LOG_N1);
+        if (LOG_N1 == 5 || logC >= 3)
+            crt32_columns<LOG_N1, LN2, VJ>(res, t.inv32 + size_t(i0) * kMaxN, logN, logC, np, s_p + i0, sA);
+        else
+            crt32_columns<LOG_N1, LN2, 1>(res, t.inv32 + size_t(i0) * kMaxN, logN, logC, np, s_p + i0, sA);
         if (g == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -656,7 +742,7 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
             const uint32_t idesc = (2u << 4) | (uint32_t(NC >> 3) << 17) | (uint32_t(kCrt32Rows >> 4) << 24);
             const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB) + uint32_t(g) * 1024u;
             for (int s = 0; s < (4 * np + 31) / 32; ++s) {
-                const uint64_t da = kmajor_desc(a0 + uint32_t(s) * 256u, 128u, 1024u);
+                const uint64_t da = kmajor_desc(a0 + uint32_t(s) * 2u * A::kChunk, A::kChunk, A::kGroup);
                 const uint64_t db = kmajor_desc(b0 + uint32_t(s) * 256u, 128u, 2048u);
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
@@ -668,30 +754,21 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
                          : "memory");
         }
     }
-    ok = __syncthreads_and(ok && mma_wait(bar_addr, uint32_t((passes - 1) & 1)) ? 1 : 0) != 0;
+    ok = __syncthreads_and(ok && (warp != 0 || mma_wait(bar_addr, uint32_t((passes - 1) & 1))) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     // every MMA has read A: it takes the output tile
     uint32_t* s_out = reinterpret_cast<uint32_t*>(sA);
     if (32 * warp < T) {
         uint32_t* o = s_out + tid * L;
-        switch (LW) {
-#define NC_CRT32_FINISH(n)                                                                                     \
-    case n:                                                                                                    \
-        if (ok)                                                                                                \
-            crt32_finish<n>(qc, s_negm, s_nq, s_q, taddr + (uint32_t(32 * warp) << 16), L, o, tid < T);         \
-        else if (tid < T)                                                                                      \
-            crt32_coeff_plain<n>(reinterpret_cast<const uint32_t*>(d.ra), qc, t.pc32, t.inv32, int(d.logN),     \
-                                 LOG_N1, k, L, tid >> logC, j0 + (tid & (C - 1)), o);                          \
-        break;
-            NC_LW_CASES(NC_CRT32_FINISH)
-#undef NC_CRT32_FINISH
-            default: break;
-        }
+        if (ok)
+            crt32_finish_any(LW, qc, s_negm, taddr + (uint32_t(32 * warp) << 16), L, o, tid < T);
+        else if (tid < T)
+            crt32_plain_any(LW, ra, qc, t.pc32, t.inv32, logN, LOG_N1, k, L, tid >> logC, j0 + (tid & (C - 1)), o);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    crt32_store(d.c, N2, L, j0, C, 1 << LOG_N1, s_out);
+    crt32_store(c_out, N2, L, j0, C, 1 << LOG_N1, s_out);
     if (!ok) mma_wait(bar_addr, uint32_t((passes - 1) & 1));  // late MMAs end before the tensor memory is given back
 }
 
@@ -839,7 +916,7 @@ template <int LOG_N1>
 __global__ void __launch_bounds__(kThreads, 4) k_batch_crt_tc32(BatchCrtArgs a, uint32_t cols) {
 #if NC_HAS_TCGEN05
     const uint2 w = __ldg(a.items + blockIdx.x);
-    const ProductDesc d = a.products[w.x].d;
+    const ProductDesc& d = a.products[w.x].d;
     crt32_cta<LOG_N1>(d, a.tables, int(w.y), crt32_batch_log_tile(int(d.logN)), cols);
 #endif
 }

@@ -69,7 +69,7 @@ __device__ __forceinline__ int swz(int x) {
 }
 
 // ------------------------------------------------------------------------------------------
-// column stages (registers), as column_forward / column_inverse of the 62-bit engine
+// column stages (registers), as column_forward / column_inverse of the 62-bit engine, of VJ columns
 
 // Twiddles (root << s) + blk and the next one: neighbours from stage 1 on, one 16-byte load.
 struct ColumnTwiddles {
@@ -87,8 +87,8 @@ __device__ __forceinline__ ColumnTwiddles column_twiddles(const uint2* tw, int a
     return r;
 }
 
-template <int LOG_N1>
-__device__ __forceinline__ void column_forward_root(const uint2* tw, int root, uint32_t p, uint32_t (&v)[1 << LOG_N1]) {
+template <int LOG_N1, int VJ>
+__device__ __forceinline__ void column_forward_root(const uint2* tw, int root, uint32_t p, uint32_t (&v)[VJ][1 << LOG_N1]) {
     constexpr int N1 = 1 << LOG_N1;
     const uint32_t p2 = 2 * p;
 #pragma unroll
@@ -102,15 +102,16 @@ __device__ __forceinline__ void column_forward_root(const uint2* tw, int root, u
 #pragma unroll
                 for (int jj = 0; jj < half; ++jj) {
                     const int u = (blk + e) * 2 * half + jj;
-                    ct_bfly(v[u], v[u + half], w.w[e].x, w.w[e].y, p, p2);
+#pragma unroll
+                    for (int c = 0; c < VJ; ++c) ct_bfly(v[c][u], v[c][u + half], w.w[e].x, w.w[e].y, p, p2);
                 }
             }
         }
     }
 }
 
-template <int LOG_N1>
-__device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, uint32_t p, uint32_t (&v)[1 << LOG_N1]) {
+template <int LOG_N1, int VJ>
+__device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, uint32_t p, uint32_t (&v)[VJ][1 << LOG_N1]) {
     constexpr int N1 = 1 << LOG_N1;
     const uint32_t p2 = 2 * p;
 #pragma unroll
@@ -124,7 +125,8 @@ __device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, u
 #pragma unroll
                 for (int jj = 0; jj < half; ++jj) {
                     const int u = (blk + e) * 2 * half + jj;
-                    gs_bfly(v[u], v[u + half], w.w[e].x, w.w[e].y, p, p2);
+#pragma unroll
+                    for (int c = 0; c < VJ; ++c) gs_bfly(v[c][u], v[c][u + half], w.w[e].x, w.w[e].y, p, p2);
                 }
             }
         }
