@@ -234,12 +234,14 @@ struct RowConfig {
 constexpr int kMaxLogN1 = 5;
 constexpr int kRowLogCap = 13;
 
+// The 62-bit engine's row configuration before any tuning: radix-8 passes on blocks of N / 8, 2^6 to
+// 2^11 residues (us a product, blocks of min(N, 2^12) with radix-16 passes against these: 434 bits,
+// N = 2048 42.3 and 23.2, N = 65536 77.3 and 74.0; 1000 bits, N = 1024 65.0 and 46.0, N = 65536 219 and
+// 178; three operands of 868 bits, N = 16384 125 and 99); radix 16 below, where radix 8 has no kernel.
 inline RowConfig default_row_config(int logN) {
-    RowConfig c{};
-    c.logN2 = logN < kRowLogMax ? logN : kRowLogMax;
-    c.logE = 4;
-    c.threads = 256;
-    return c;
+    if (logN < 6) return RowConfig{logN, 4, 256};
+    const int block = logN - 3;
+    return RowConfig{block < 6 ? 6 : block > 11 ? 11 : block, 3, 256};
 }
 
 // Geometry of one product under a row configuration.

@@ -293,8 +293,10 @@ bool word64_forced() {
 }
 
 // Row configuration of the 30-bit engine before any tuning: blocks of 2^11 with radix-8 passes
-// where N allows them, else the largest radix-16 block.
+// where N allows them, else the largest radix-16 block; blocks of 2^12 at N = 2^16, whose columns would
+// have 32 points otherwise (868 bits: 74.7 us a product against 82.8; N = 2^15: 43.1 against 41.0).
 RowConfig default_row_config32(int logN) {
+    if (logN == kMaxLogN) return RowConfig{12, 3, 512};
     RowConfig c{logN < 11 ? logN : 11, 3, 256};
     if (!row_config_valid(logN, c) || !row32_kernel(c)) c = RowConfig{logN < kRowLogMax ? logN : kRowLogMax, 4, 256};
     return c;

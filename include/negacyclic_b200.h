@@ -191,7 +191,8 @@ int nc_plan_get_row_config(const nc_plan* plan, int* log_block, int* log_radix, 
    (nc_plan_set_residue_engine / nc_plan_set_crt_engine to the integer pipes select the 62-bit
    engine). Row configurations (nc_plan_set_row_config / get) apply to the engine in use;
    nc_row_variants32 lists the 30-bit engine's as nc_row_variants lists the 62-bit one's. Batches,
-   servers, chained products and nc_multiply_device_noalloc run the 62-bit engine.
+   servers and nc_multiply_device_noalloc follow the plan's engine (the last where both operands'
+   residues fit its fixed scratch); chained products run the 62-bit engine.
    nc_plan_word_bits returns 32 or 64 (the engine in use) and writes its prime count to k (may be
    NULL); nc_plan_set_word_bits fails with NC_EINVAL where the 30-bit engine cannot run. Both
    engines give the same product. Set it only while no product of the plan is in flight. */
