@@ -168,11 +168,12 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
                              smem_u32(&bar))
                          : "memory");
         }
-        const bool ok = !failed && mma_wait(smem_u32(&bar), uint32_t(g & 1));
+        // one warp polls, the others wait at the barrier
+        const bool ok = __syncthreads_and(warp != 0 || (!failed && mma_wait(smem_u32(&bar), uint32_t(g & 1))) ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int ib = i0 + 8 * half;
         const int ie = i0 + np < ib + 8 ? i0 + np : ib + 8;
-        if (__all_sync(0xffffffffu, ok)) {
+        if (ok) {
             const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16);
             for (int i = ib; i < ie; i += 2) {
                 uint32_t s[16];
@@ -204,7 +205,8 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        failed = __syncthreads_or(ok ? 0 : 1) != 0;  // also: this pass's reads are done before the next MMA
+        failed = !ok;
+        __syncthreads();  // this pass's reads are done before the next MMA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (warp == 0)

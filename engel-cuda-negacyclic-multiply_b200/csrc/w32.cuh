@@ -28,11 +28,22 @@ __device__ __forceinline__ uint32_t shoup(uint32_t y, uint32_t w, uint32_t wq, u
     return y * w - __umulhi(y, wq) * p;
 }
 
+// Zero that the compiler cannot see (p < 2^31). A sum with it as third operand is one three-input
+// addition; the compiler issues most two-input ones as multiply-adds with a factor of one, on the multiply
+// pipe, which the row stage keeps busiest (1.5 of 4.5 multiply-adds a butterfly; 64 x 16384: that pipe
+// 69% -> 59% busy, 861 -> 848 us a batch).
+__device__ __forceinline__ uint32_t hidden_zero(uint32_t p) {
+    uint32_t z;
+    asm("and.b32 %0, %1, 0x80000000;" : "=r"(z) : "r"(p));
+    return z;
+}
+
 // Forward butterfly (x, y) -> (x + w y, x - w y); inputs and outputs in [0, 4p).
-__device__ __forceinline__ void ct_bfly(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wq, uint32_t p, uint32_t p2) {
+__device__ __forceinline__ void ct_bfly(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wq, uint32_t p, uint32_t p2,
+                                        uint32_t z = 0) {
     const uint32_t u = csub(x, p2);
     const uint32_t t = shoup(y, w, wq, p);
-    x = u + t;
+    x = u + t + z;
     y = u - t + p2;
 }
 
@@ -46,8 +57,9 @@ __device__ __forceinline__ void gs_bfly(uint32_t& x, uint32_t& y, uint32_t w, ui
 
 // The inverse butterfly with twiddle -w: (x, y) -> (x + y, (y - x) w). The row stage's inverse
 // twiddles are negated forward ones (below), so it takes the forward pair unchanged.
-__device__ __forceinline__ void gs_bfly_neg(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wq, uint32_t p, uint32_t p2) {
-    const uint32_t s = csub(x + y, p2);
+__device__ __forceinline__ void gs_bfly_neg(uint32_t& x, uint32_t& y, uint32_t w, uint32_t wq, uint32_t p, uint32_t p2,
+                                            uint32_t z) {
+    const uint32_t s = csub(x + y + z, p2);
     const uint32_t d = y - x + p2;
     x = s;
     y = shoup(d, w, wq, p);
@@ -136,6 +148,31 @@ __device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, u
 // ------------------------------------------------------------------------------------------
 // row blocks: the register passes of stages.cuh over u32 residues
 
+// Element of register slot e in pass PASS for thread lt, as row_index of stages.cuh, but for a last pass
+// of fewer stages: the thread's groups there are neighbours. In every pass after the first a block of
+// N2 >> l0 elements then belongs to the same run of threads as in the pass before.
+template <class S, int PASS>
+__host__ __device__ __forceinline__ constexpr int row_index(int lt, int e) {
+    constexpr int R = S::r(PASS), LL = S::lolog(PASS);
+    if (R < S::LE) return lt * S::E + e;
+    const int hi = lt >> LL, lo = lt & ((1 << LL) - 1);
+    return (hi << (S::LOG_N2 - S::l0(PASS))) + (e << LL) + lo;
+}
+
+// Barrier of the threads that share a block of pass PASS, whose values the exchanges after it move: a warp,
+// part of the CTA, or all of it. With CTA barriers alone an item had 18; now five are wider than a warp
+// (blocks of 2^11, 256 threads).
+template <class S, int PASS>
+__device__ __forceinline__ void block_sync() {
+    constexpr int D = S::T >> S::l0(PASS);
+    if constexpr (D <= 32)
+        __syncwarp();
+    else if constexpr (D >= 256)
+        __syncthreads();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + int(threadIdx.x) / D), "n"(D) : "memory");
+}
+
 // One pass of R stages over the thread's groups. tw is a row block's staged twiddles (local
 // stage l at tw[(1 << l) + t], stage_twiddles). Forward passes take entry t of the row block's
 // forward table; inverse passes take the staged forward twiddles of the mirrored row block in
@@ -146,11 +183,10 @@ __device__ __forceinline__ void column_inverse_root(const uint2* tw, int root, u
 template <class S, int PASS, bool FWD>
 __device__ __forceinline__ void row_pass(uint32_t (&v)[S::E], const uint2* tw, int lt, uint32_t p) {
     constexpr int R = S::r(PASS), LL = S::lolog(PASS), L0 = S::l0(PASS);
-    const uint32_t p2 = 2 * p;
+    const uint32_t p2 = 2 * p, z = hidden_zero(p);
 #pragma unroll
     for (int q = 0; q < (S::E >> R); ++q) {
-        const int g = lt + S::T * q;
-        const int hi = g >> LL;
+        const int hi = R < S::LE ? (lt << (S::LE - R)) + q : lt >> LL;
 #pragma unroll
         for (int jj = 0; jj < R; ++jj) {
             const int j = FWD ? jj : R - 1 - jj;
@@ -189,58 +225,72 @@ __device__ __forceinline__ void row_pass(uint32_t (&v)[S::E], const uint2* tw, i
                 for (int s0 = 0; s0 < half; ++s0) {
                     const int e = q * (1 << R) + blk * 2 * half + s0;
                     if (FWD)
-                        ct_bfly(v[e], v[e + half], w[blk].x, w[blk].y, p, p2);
+                        ct_bfly(v[e], v[e + half], w[blk].x, w[blk].y, p, p2, z);
                     else
-                        gs_bfly_neg(v[e], v[e + half], w[blk].x, w[blk].y, p, p2);
+                        gs_bfly_neg(v[e], v[e + half], w[blk].x, w[blk].y, p, p2, z);
                 }
             }
         }
     }
 }
 
-// A thread's values of pass PASS to / from the row buffer. When the pass's groups are runs of
-// consecutive elements (lolog 0), each run of four (or two) goes as one 16-byte (8-byte) access.
+// Place of element x in a row buffer. Blocks of up to 2^11 (whose CTAs have the room) are padded by four
+// words after every 32: the bits of a thread's element and of its register slot are disjoint, so the
+// place is a sum and every access of a pass is one base register and a constant offset. Blocks of 2^12
+// are XOR-swizzled (one logic operation an access). Both keep the passes' accesses on distinct banks.
+template <class S>
+struct RowPlace {
+    static constexpr bool kPadded = S::LOG_N2 >= 5 && S::LOG_N2 <= 11;
+    static constexpr int kWords = kPadded ? S::N2 + S::N2 / 8 : S::N2;
+    __host__ __device__ static constexpr int pad(int x) { return kPadded ? x + ((x >> 5) << 2) : x; }
+    // base: the place of the thread's slot 0; slot: row_index of the slot for thread 0
+    __device__ static int base(int x) { return kPadded ? pad(x) : swz(x); }
+    __device__ static int at(int base, int slot) { return kPadded ? base + pad(slot) : base ^ swz(slot); }
+};
+
+// A thread's values of pass PASS to / from the row buffer. In a last pass (lolog 0) they are consecutive
+// elements and go four (or two) at a time.
 template <class S, int PASS>
 __device__ __forceinline__ void row_store(const uint32_t (&v)[S::E], uint32_t* buf, int lt) {
-    if constexpr (S::lolog(PASS) == 0 && S::r(PASS) >= 2) {
+    using P = RowPlace<S>;
+    const int b = P::base(row_index<S, PASS>(lt, 0));
+    if constexpr (S::lolog(PASS) == 0 && S::E >= 4) {
 #pragma unroll
-        for (int e = 0; e < S::E; e += 4) {
-            const int x = row_index<S, PASS>(lt, e);
-            reinterpret_cast<uint4*>(buf)[swz(x) >> 2] = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
-        }
-    } else if constexpr (S::lolog(PASS) == 0 && S::r(PASS) == 1) {
+        for (int e = 0; e < S::E; e += 4)
+            *reinterpret_cast<uint4*>(buf + P::at(b, row_index<S, PASS>(0, e))) = make_uint4(v[e], v[e + 1], v[e + 2], v[e + 3]);
+    } else if constexpr (S::lolog(PASS) == 0) {
 #pragma unroll
-        for (int e = 0; e < S::E; e += 2) {
-            const int x = row_index<S, PASS>(lt, e);
-            reinterpret_cast<uint2*>(buf)[swz(x) >> 1] = make_uint2(v[e], v[e + 1]);
-        }
+        for (int e = 0; e < S::E; e += 2)
+            *reinterpret_cast<uint2*>(buf + P::at(b, row_index<S, PASS>(0, e))) = make_uint2(v[e], v[e + 1]);
     } else {
 #pragma unroll
-        for (int e = 0; e < S::E; ++e) buf[swz(row_index<S, PASS>(lt, e))] = v[e];
+        for (int e = 0; e < S::E; ++e) buf[P::at(b, row_index<S, PASS>(0, e))] = v[e];
     }
 }
 
 template <class S, int PASS>
 __device__ __forceinline__ void row_load(uint32_t (&v)[S::E], const uint32_t* buf, int lt) {
-    if constexpr (S::lolog(PASS) == 0 && S::r(PASS) >= 2) {
+    using P = RowPlace<S>;
+    const int b = P::base(row_index<S, PASS>(lt, 0));
+    if constexpr (S::lolog(PASS) == 0 && S::E >= 4) {
 #pragma unroll
         for (int e = 0; e < S::E; e += 4) {
-            const uint4 q = reinterpret_cast<const uint4*>(buf)[swz(row_index<S, PASS>(lt, e)) >> 2];
+            const uint4 q = *reinterpret_cast<const uint4*>(buf + P::at(b, row_index<S, PASS>(0, e)));
             v[e] = q.x;
             v[e + 1] = q.y;
             v[e + 2] = q.z;
             v[e + 3] = q.w;
         }
-    } else if constexpr (S::lolog(PASS) == 0 && S::r(PASS) == 1) {
+    } else if constexpr (S::lolog(PASS) == 0) {
 #pragma unroll
         for (int e = 0; e < S::E; e += 2) {
-            const uint2 q = reinterpret_cast<const uint2*>(buf)[swz(row_index<S, PASS>(lt, e)) >> 1];
+            const uint2 q = *reinterpret_cast<const uint2*>(buf + P::at(b, row_index<S, PASS>(0, e)));
             v[e] = q.x;
             v[e + 1] = q.y;
         }
     } else {
 #pragma unroll
-        for (int e = 0; e < S::E; ++e) v[e] = buf[swz(row_index<S, PASS>(lt, e))];
+        for (int e = 0; e < S::E; ++e) v[e] = buf[P::at(b, row_index<S, PASS>(0, e))];
     }
 }
 
@@ -248,9 +298,9 @@ template <class S, int PASS>
 __device__ __forceinline__ void row_forward_from(uint32_t (&v)[S::E], uint32_t* buf, const uint2* tw, int lt, uint32_t p) {
     row_pass<S, PASS, true>(v, tw, lt, p);
     if constexpr (PASS + 1 < S::NPASS) {
-        __syncthreads();
+        block_sync<S, PASS>();
         row_store<S, PASS>(v, buf, lt);
-        __syncthreads();
+        block_sync<S, PASS>();
         row_load<S, PASS + 1>(v, buf, lt);
         row_forward_from<S, PASS + 1>(v, buf, tw, lt, p);
     }
@@ -260,9 +310,9 @@ template <class S, int PASS>
 __device__ __forceinline__ void row_inverse_from(uint32_t (&v)[S::E], uint32_t* buf, const uint2* tw, int lt, uint32_t p) {
     row_pass<S, PASS, false>(v, tw, lt, p);
     if constexpr (PASS > 0) {
-        __syncthreads();
+        block_sync<S, PASS>();  // the values there were read in this pass's blocks
         row_store<S, PASS>(v, buf, lt);
-        __syncthreads();
+        block_sync<S, PASS - 1>();
         row_load<S, PASS - 1>(v, buf, lt);
         row_inverse_from<S, PASS - 1>(v, buf, tw, lt, p);
     }
@@ -272,17 +322,19 @@ __device__ __forceinline__ void row_inverse_from(uint32_t (&v)[S::E], uint32_t* 
 // 256-thread ones (four per SM) have no room left for it.
 NC_HD constexpr bool row_prefetch_b(int threads) { return threads == 512; }
 
-// Dynamic shared memory of a row CTA: the row buffer, the buffer of operand a's transform and,
-// with row_prefetch_b, b's residue block (4 bytes a residue each), then each row block's forward
-// and inverse twiddles (8 bytes an entry, N2 entries each).
+// Dynamic shared memory of a row CTA: the row buffer and the buffer of operand a's transform (4 bytes a
+// residue each, an eighth more where padded: blocks of up to 2^11, 256 threads) and, with
+// row_prefetch_b, b's residue block, then each row block's forward and inverse twiddles (8 bytes an
+// entry, N2 entries each).
 NC_HD constexpr size_t row_smem_bytes(int threads, int logE) {
-    return size_t(threads) * (size_t(1) << logE) * (row_prefetch_b(threads) ? 28 : 24);
+    return size_t(threads) * (size_t(1) << logE) * (row_prefetch_b(threads) ? 28 : 25);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // Bounded wait for phase `parity` of the mbarrier at shared address `bar`: false if it did not
-// complete within 2^22 polls.
+// complete within 2^22 polls. cta_wait is the whole CTA's: one warp polls and the rest wait at the
+// barrier (every warp polling took a sixth of the row kernel's instructions).
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
     for (uint32_t it = 0; it < (1u << 22); ++it) {
         uint32_t done;
@@ -296,6 +348,10 @@ __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
         if (done) return true;
     }
     return false;
+}
+
+__device__ __forceinline__ bool cta_wait(uint32_t bar, uint32_t parity) {
+    return __syncthreads_and(threadIdx.x >= 32 || bar_wait(bar, parity) ? 1 : 0) != 0;
 }
 
 // The twiddles of the row block under node `base` of the merged tree: local stage l uses the 2^l
@@ -369,11 +425,13 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
     const int base_mirror = (2 << logN1) - 1 - u;
     const size_t off = size_t(i) * N + size_t(u) * S::N2;
     constexpr bool PF_B = row_prefetch_b(THREADS);
-    constexpr int NBUF = PF_B ? 3 : 2;
-    uint32_t* buf = reinterpret_cast<uint32_t*>(smem) + rr * S::N2;
-    uint32_t* buf_a = reinterpret_cast<uint32_t*>(smem) + size_t(ROWS) * S::N2 + rr * S::N2;
+    using P = RowPlace<S>;
+    static_assert(!(PF_B && P::kPadded), "no room for padded buffers beside b's block");
+    uint32_t* buf = reinterpret_cast<uint32_t*>(smem) + rr * P::kWords;
+    uint32_t* buf_a = reinterpret_cast<uint32_t*>(smem) + size_t(ROWS) * P::kWords + rr * P::kWords;
     uint32_t* b_in = reinterpret_cast<uint32_t*>(smem) + size_t(2) * ROWS * S::N2 + rr * S::N2;  // with PF_B
-    uint2* s_twf = reinterpret_cast<uint2*>(smem + size_t(NBUF) * ROWS * S::N2 * 4) + size_t(rr) * 2 * S::N2;
+    uint2* s_twf = reinterpret_cast<uint2*>(smem + size_t(ROWS) * (2 * P::kWords + (PF_B ? S::N2 : 0)) * 4) +
+                   size_t(rr) * 2 * S::N2;
     uint2* s_twi = s_twf + S::N2;
     const uint2* twf = t.fwd32 + size_t(i) * kMaxN;
     const uint32_t* ra = reinterpret_cast<const uint32_t*>(d.ra);
@@ -389,11 +447,11 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
         stage_twiddles<LOG_N2>(twf, base, s_twf, bar);
         if (inverse) stage_twiddles<LOG_N2>(twf, base_mirror, s_twi, bar);
     }
-    // every thread waits for the copies (bounded); if any gave up, each row's threads copy its
+    // the CTA waits for the copies (bounded); if that gave up, each row's threads copy its
     // twiddles themselves and, before the item ends, wait once more for the copies in flight
     bool staged = use_bulk;
     auto twiddles_ready = [&] {
-        if (use_bulk) staged = __syncthreads_and(bar_wait(bar, parity) ? 1 : 0) != 0;
+        if (use_bulk) staged = cta_wait(bar, parity);
         if (!staged) {
             copy_twiddles<LOG_N2>(twf, base, s_twf, lt, S::T);
             if (inverse) copy_twiddles<LOG_N2>(twf, base_mirror, s_twi, lt, S::T);
@@ -460,7 +518,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
         }
         __syncthreads();
 #pragma unroll
-        for (int e = 0; e < S::E; ++e) buf_a[swz(row_index<S, 0>(lt, e))] = av[e];
+        for (int e = 0; e < S::E; ++e) buf_a[P::at(P::base(row_index<S, 0>(lt, 0)), row_index<S, 0>(0, e))] = av[e];
     } else {
 #pragma unroll
         for (int e = 0; e < S::E; ++e) v[e] = buf_a[row_index<S, 0>(lt, e)];
@@ -488,7 +546,8 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
         }
     }
     row_forward_from<S, 0>(v, buf, s_twf, lt, p);
-    __syncthreads();
+    // a's transform was written by this thread, or (cached) before the barriers of b's first exchange
+    if constexpr (S::NPASS == 1) __syncthreads();
     const uint32_t p2 = 2 * p;
     uint32_t av[S::E];
     row_load<S, LAST>(av, buf_a, lt);
@@ -530,8 +589,8 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
     const int u0 = rb0 & ((1 << logN1) - 1), u1 = rb1 & ((1 << logN1) - 1);
     const uint32_t p = __ldg(&t.pc32[i].p), pinv = __ldg(&t.pc32[i].pinv);
     uint32_t* buf = reinterpret_cast<uint32_t*>(smem);
-    uint32_t* buf_a = buf + S::N2;
-    uint2* const s_tw0 = reinterpret_cast<uint2*>(smem + size_t(2) * S::N2 * 4);
+    uint32_t* buf_a = buf + RowPlace<S>::kWords;
+    uint2* const s_tw0 = reinterpret_cast<uint2*>(smem + size_t(2) * RowPlace<S>::kWords * 4);
     uint2* const s_tw1 = s_tw0 + S::N2;
     const uint2* twf = t.fwd32 + size_t(i) * kMaxN;
     const uint32_t* ra = reinterpret_cast<const uint32_t*>(d.ra);
@@ -566,7 +625,7 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
     }
     // phase whose copies may still be in flight (-1: none) once a wait gave up
     int pending = -1;
-    bool staged = use_bulk && __syncthreads_and(bar_wait(bar, parity) ? 1 : 0) != 0;
+    bool staged = use_bulk && cta_wait(bar, parity);
     if (!staged) {
         if (use_bulk) pending = 0;
         copy_twiddles<LOG_N2>(twf, (1 << logN1) + u0, s_tw0, lt, S::T);
@@ -580,11 +639,11 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
         const size_t off = j ? off1 : off0;
         if (j == 1) {
             if (staged) {
-                staged = __syncthreads_and(bar_wait(bar, parity ^ 1u) ? 1 : 0) != 0;
+                staged = cta_wait(bar, parity ^ 1u);
                 if (!staged) pending = 1;
             } else if (pending == 0) {
                 // once the late copies of the first member are done, its buffers are free
-                if (__syncthreads_and(bar_wait(bar, parity) ? 1 : 0) != 0)
+                if (cta_wait(bar, parity))
                     pending = -1;
                 else if (error && lt == 0 && atomicCAS(error, 0u, 1u) == 0u)
                     error[1] = what;
@@ -603,9 +662,8 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
 #pragma unroll
         for (int e = 0; e < S::E; ++e) v[e] = __ldcg(rbr + off + row_index<S, 0>(lt, e));
         row_forward_from<S, 0>(v, buf, j ? s_tw1 : s_tw0, lt, p);
-        __syncthreads();
         {
-            uint32_t av[S::E];
+            uint32_t av[S::E];  // written by this thread
             row_load<S, LAST>(av, buf_a, lt);
 #pragma unroll
             for (int e = 0; e < S::E; ++e) v[e] = mont(csub(csub(av[e], p2), p), v[e], p, pinv);
