@@ -73,7 +73,8 @@ __device__ __forceinline__ int res_slot(int i, int x, int C) { return x ^ ((i * 
 // `taddr_slot` are the CTA's mbarrier and tensor-memory address slot in shared memory.
 template <int LOG_N1>
 __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& t, int operand, int tile, uint8_t* smem,
-                                            uint64_t& bar, uint32_t& taddr_slot) {
+                                            uint64_t (&bars)[2], uint32_t& taddr_slot) {
+    uint64_t& bar = bars[0];
     constexpr int N1 = 1 << LOG_N1;
     const int N = 1 << d.logN;
     const int N2 = N >> LOG_N1;
@@ -97,8 +98,17 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
+        for (int e = 0; e < 2; ++e)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[e])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // B: the weight bytes of the first `groups` primes, already in shared-memory order, as one copy
+        // that the thread of the MMAs waits for
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bars[1])), "r"(groups * 1024)
+                     : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(sB)),
+                     "l"(t.res_w), "r"(groups * 1024), "r"(smem_u32(&bars[1]))
+                     : "memory");
     }
     // The next kernel on the stream may be scheduled only once every CTA of this one holds its
     // tensor memory: a dependent that allocates before its griddepcontrol.wait could otherwise
@@ -106,8 +116,6 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     __syncthreads();
     pdl_trigger();
 
-    // B: the weight bytes of the first `groups` primes, already in shared-memory order
-    for (int q = tid; q < groups * 64; q += kThreads) cp_async16(sB + q * 16, t.res_w + q);
     for (int w = tid; w < k; w += kThreads) s_p[w] = __ldg(t.primes + w);
     pdl_wait();  // the operand and the residue rows belong to the stream's previous kernels
     // A: 16-byte chunk q = (row group, K chunk, row), row m = u C + j is coefficient u N2 + j0 + j
@@ -137,7 +145,9 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> MMA reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    // (the thread of the MMAs has also waited for the weights; if that gave up, the residues go by the
+    // integer pipes)
+    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     const int slices = (kbytes + 31) / 32;
@@ -146,7 +156,6 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     // and half w / 4 of the pass's primes
     const int m = 32 * (warp & 3) + lane;
     const int half = warp >> 2;
-    bool failed = false;
     for (int g = 0; g * kDecTcPassPrimes < k; ++g) {
         const int i0 = g * kDecTcPassPrimes;
         const int np = k - i0 < kDecTcPassPrimes ? k - i0 : kDecTcPassPrimes;
@@ -279,7 +288,7 @@ template <int LOG_N1>
 __global__ void NC_DEC_TC_BOUNDS(LOG_N1) k_dec_tc(ProductDesc d, Tables t, int first_operand, int tile0, int tiles) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t taddr_slot;
     dec_tc_item<LOG_N1>(d, t, first_operand + int(blockIdx.x) / tiles, tile0 + int(blockIdx.x) % tiles, smem, bar,
                         taddr_slot);
@@ -292,7 +301,7 @@ template <int LOG_N1>
 __global__ void NC_DEC_TC_BOUNDS(LOG_N1) k_batch_dec_tc(BatchCrtArgs a) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t taddr_slot;
     const uint2 w = __ldg(a.items + blockIdx.x);
     const BatchProduct& bp = a.products[w.x];

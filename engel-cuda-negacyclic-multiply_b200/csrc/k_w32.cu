@@ -36,6 +36,14 @@ __device__ __forceinline__ void cp_async4(void* dst, const void* src, uint32_t s
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
                  : "memory");
 }
+// One thread: `bytes` (a multiple of 16) to shared memory by a bulk copy that completes phase 0 of `bar`.
+__device__ __forceinline__ void bulk_table(void* dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
 __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c) {
     uint64_t d;
     asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
@@ -181,7 +189,8 @@ __device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, con
 // offsets are then constants), else 0. Primes [i0, i1), i0 a multiple of 32.
 template <int LOG_N1, int CC, int LN2>
 __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables& t, int operand, int tile, int i0,
-                                              int i1, uint8_t* smem, uint64_t& bar, uint32_t& taddr_slot) {
+                                              int i1, uint8_t* smem, uint64_t (&bars)[2], uint32_t& taddr_slot) {
+    uint64_t& bar = bars[0];
     const int N = 1 << d.logN;
     const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
     const int T = CC ? kDecTcRows : (N < kDecTcRows ? N : kDecTcRows);
@@ -205,12 +214,13 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     }
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bars[1])) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        // the weights, already in shared-memory order, as one copy that the thread of the MMAs waits for
+        bulk_table(sB, t.res_w32 + size_t(i0 >> 1) * 64, uint32_t(wpairs) * 1024u, smem_u32(&bars[1]));
     }
     __syncthreads();
 
-    const uint4* w_src = t.res_w32 + size_t(i0 >> 1) * 64;
-    for (int q = tid; q < wpairs * 64; q += kThreads) cp_async16(sB + q * 16, w_src + q);
     for (int w = tid; w < 2 * wpairs; w += kThreads) {
         const PrimeConst32 pc = t.pc32[i0 + w];  // the MMAs' primes
         s_pc[w] = make_uint2(pc.p, pc.bar >> 2);
@@ -247,7 +257,9 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    // (the thread of the MMAs has also waited for the weights; if that gave up, the residues go by the
+    // integer pipes)
+    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     const int slices = (kbytes + 31) / 32;
@@ -260,7 +272,6 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     int slot[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) slot[e] = CC ? res_slot(e, m, CC) : 0;
-    bool failed = false;
     for (int g = 0; g * kDecTc32PassPrimes < k; ++g) {
         const int ig = g * kDecTc32PassPrimes;
         const int np = k - ig < kDecTc32PassPrimes ? k - ig : kDecTc32PassPrimes;
@@ -334,7 +345,7 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
 // The item by its tile width and row length.
 template <int LOG_N1>
 __device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables& t, int operand, int tile, int i0, int i1,
-                                             uint8_t* smem, uint64_t& bar, uint32_t& taddr_slot) {
+                                             uint8_t* smem, uint64_t (&bar)[2], uint32_t& taddr_slot) {
     if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
         dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 12>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
     else if (d.logN >= 7)
@@ -351,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
                                                            int tiles, int split) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t taddr_slot;
     int b = int(blockIdx.x), i0 = 0, i1 = int(d.k);
     if (split) {
@@ -676,11 +687,12 @@ __device__ __forceinline__ void crt32_store(uint32_t* c, int N2, int L, int j0, 
 }
 
 // One tile with every thread of a 256-thread CTA, columns of 2^LOG_N1 points at stride 2^LN2 (N / N1
-// with LN2 0). The caller owns tensor-memory columns for the product's LW at `taddr` and an
-// initialised mbarrier `bar`.
+// with LN2 0). The caller owns tensor-memory columns for the product's LW at `taddr` and
+// two initialised mbarriers `bars` (the MMAs', the table's).
 template <int LOG_N1, int LN2>
 __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
-                                                uint8_t* smem, uint32_t taddr, uint64_t* bar) {
+                                                uint8_t* smem, uint32_t taddr, uint64_t* bars) {
+    uint64_t* bar = bars;
     using A = Crt32Layout<LOG_N1>;
     // the descriptor's fields once (a batch's lies in global memory)
     const int LW = int(d.LW), NC = crt32_cols(LW), logN = int(d.logN);
@@ -708,12 +720,9 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
         s_nq[w] = __ldg(qc->neg_q + w);
         s_q[w] = __ldg(qc->q + w);
     }
-    // the table is first read by the MMAs: its copy runs behind the column stages (the K chunks
-    // that the last slice reads; its K bytes from 4 k up are zero, so A's are never read into the sums)
-    const int slices_all = (4 * k + 31) / 32;
-    for (int w = tid; w < NC * 16; w += kThreads)
-        if (((w >> 3) & 15) < 2 * slices_all) cp_async16(sB + 16 * w, d.crt_b + w);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    // the table is first read by the MMAs: its copy runs behind the column stages, and the thread that
+    // issues them waits for it (its K bytes from 4 k up are zero, so A's are never read into the sums)
+    if (tid == 0) bulk_table(sB, d.crt_b, uint32_t(NC) * 256u, smem_u32(bars + 1));
     __syncthreads();
     pdl_wait();  // the residues come from the stream's previous kernel
     pdl_trigger();
@@ -721,6 +730,7 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
     const uint32_t bar_addr = smem_u32(bar);
     const int passes = (k + 31) >> 5;
     bool ok = true;
+    int issued = 0;  // passes whose MMAs have been issued
 #pragma unroll 1
     for (int g = 0; g < passes; ++g) {
         // the A buffer is free once the pass before has been read
@@ -733,10 +743,14 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
             crt32_columns<LOG_N1, LN2, VJ>(res, t.inv32 + size_t(i0) * kMaxN, logN, logC, np, s_p + i0, sA);
         else
             crt32_columns<LOG_N1, LN2, 1>(res, t.inv32 + size_t(i0) * kMaxN, logN, logC, np, s_p + i0, sA);
-        if (g == 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
+        if (g == 0)
+            ok = __syncthreads_and(tid != 0 || mma_wait(smem_u32(bars + 1), 0) ? 1 : 0) != 0;
+        else
+            __syncthreads();
+        if (!ok) break;
+        ++issued;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (tid == 0) {
             const uint32_t idesc = (2u << 4) | (uint32_t(NC >> 3) << 17) | (uint32_t(kCrt32Rows >> 4) << 24);
@@ -769,14 +783,18 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     crt32_store(c_out, N2, L, j0, C, 1 << LOG_N1, s_out);
-    if (!ok) mma_wait(bar_addr, uint32_t((passes - 1) & 1));  // late MMAs end before the tensor memory is given back
+    if (!ok) {
+        // late copies and MMAs end (bounded) before the memory they write is given back
+        mma_wait(smem_u32(bars + 1), 0);
+        if (issued > 0) mma_wait(bar_addr, uint32_t((issued - 1) & 1));
+    }
 }
 
 // The tile within a kernel: tensor memory (`cols` columns) and the mbarrier around it.
 template <int LOG_N1>
 __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t, int tile, int logT, uint32_t cols) {
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bars[2];  // the MMAs', the table's
     __shared__ uint32_t taddr_slot;
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&taddr_slot)),
@@ -785,7 +803,8 @@ __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t,
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
+        for (int e = 0; e < 2; ++e)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + e)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -793,9 +812,9 @@ __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t,
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
-        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, smem, taddr, &bar);
+        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, smem, taddr, bars);
     else
-        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, smem, taddr, &bar);
+        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, smem, taddr, bars);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32)
@@ -839,7 +858,7 @@ template <int LOG_N1>
 __global__ void __launch_bounds__(kThreads, 4) k_batch_dec_tc32(BatchCrtArgs a) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar[2];
     __shared__ uint32_t taddr_slot;
     const uint2 w = __ldg(a.items + blockIdx.x);
     const BatchProduct& bp = a.products[w.x];
