@@ -119,7 +119,8 @@ struct Plan {
     bool res_tc = true;              // plain path: residue stage on the tensor cores
     // The 30-bit word engine for the plain path of a pair (k32 primes below 2^30): available with
     // tensor cores when the bound fits 64 primes; in use while `w32` is set and both tensor-core
-    // stages are selected. Batches, chains and the allocation-free entry run the 62-bit engine.
+    // stages are selected. Batches and the allocation-free entry (where both operands' residues fit
+    // its array) follow it; chains run the 62-bit engine.
     bool w32_ok = false;
     bool w32 = false;
     int k32 = 0;

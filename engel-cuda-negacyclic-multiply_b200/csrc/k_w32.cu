@@ -354,6 +354,12 @@ __device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables&
         dec_tc32_item<LOG_N1, 0, 0>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
 }
 
+// What bounds it: issue slots (the five-instruction fold of every residue, the column butterflies)
+// and the latency of a tile's phases, which four CTAs an SM overlap in part; DRAM and the tensor cores
+// are idle most of the time. Two operands of N = 65536, 868 bits: 34.8 -> 26.1 us (a fold of five
+// instructions, neighbouring columns a thread, one polling warp, one bulk copy of
+// the weights).
+//
 // Four CTAs per SM, as k_dec_tc (tensor memory holds four of 128 columns). With `split`, a CTA takes
 // one pass of 32 primes of its tile instead of all of them (small grids: every pass is then a CTA
 // of its own).
@@ -390,6 +396,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
 // What bounds it: the column butterflies and loads (59 residues of a coefficient against one
 // contraction row), so integer issue and load latency, not the tensor cores. 128-coefficient tiles
 // with the primes in passes of 32 through one 20 KB A buffer keep a CTA at 54 KB, four per SM.
+// N = 65536, 868 bits: 24.6 -> 20.5 us a stage; N = 1024, where the old CRT was a chain of 59 dependent
+// loads a thread in four CTAs: 32.8 -> 16.0 us a product.
 
 // A: [16 row groups][8 K chunks of four primes][8 rows][16 B], the chunks 16 or 32 bytes and the row
 // groups 16 bytes further apart than packed: a warp's four-byte stores (eight groups of neighbouring
@@ -831,8 +839,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables 
 // ------------------------------------------------------------------------------------------
 // row blocks
 
-// Resident CTAs per SM: radix-8 passes in 256-thread CTAs at four (64 registers; at N = 2^16,
-// k = 59: 40.0 us, against 39.9 at three and 40.9 at five), radix 16 at three.
+// What bounds it: the 32-bit multiply pipe in bursts (about 60% of cycles), and between them the waits
+// for the staged twiddles and residues and for the other warps of a block. N = 65536, 868 bits,
+// blocks of 4096: 47.3 -> 44.8 us (padded places, block barriers, additions off the multiply pipe).
+// Resident CTAs per SM: radix-8 passes in 256-thread CTAs at four (64 registers: three and five CTAs
+// are no faster at N = 2^16), radix 16 at three.
 template <int LOG_N2, int LOG_E, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3) : 2)) k_row32(ProductDesc d, Tables t) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -871,7 +882,9 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_dec_tc32(BatchCrtArgs a) 
 // Row items (x = product, y = row-CTA index) with row blocks of 2^LOG_N2, radix 8, 256 threads:
 // persistent CTAs take items in queue order; each item's twiddles and residue blocks arrive on the
 // CTA's mbarrier, one phase per item. If a bulk wait gives up (the item then loads its data with
-// plain loads), the CTA's later items use plain loads too.
+// plain loads), the CTA's later items use plain loads too. Bound as k_row32 is, without its last wave
+// (64 x 16384, 868 bits: 481 -> 437 us with padded places, block barriers and additions off the
+// multiply pipe).
 template <int LOG_N2>
 __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];

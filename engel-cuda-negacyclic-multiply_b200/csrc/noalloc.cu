@@ -13,7 +13,7 @@
 // 2 * k * N words, so the limit is k * N <= 2^19: N <= 16384 at an 868-bit q (k = 29), N <= 32768 at
 // a 434-bit q (k = 15). Larger products are rejected with NC_EINVAL. Products of a plan on the
 // 30-bit engine run on it where its 2 * k32 * N u32 fit too (all of the above but a modulus that needs
-// an odd prime more): N = 2048, 434 bits: 42.2 us a call on the 62-bit engine, 13.1 us on this one.
+// an odd prime more): N = 2048, 434 bits: 42.2 us a call on the 62-bit engine, 11.8 us on this one.
 //
 // Sharing: every call, from every plan and every stream, uses the same array and it keeps the
 // last call's contents. Nothing in it needs to start at zero (each stage writes every residue

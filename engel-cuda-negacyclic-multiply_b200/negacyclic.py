@@ -246,7 +246,8 @@ class Plan:
     def multiply_device_noalloc(self, d_a: int, d_b: int, d_c: int, stream: int = 0) -> None:
         """Like multiply_device, but allocates nothing: for callers that must not allocate device
         memory at call time. Its residue scratch is one 8 MiB array inside the library shared by
-        all calls (so overlapping calls race); limit k * N <= 2^19 (N <= 16384 at an 868-bit q)."""
+        all calls (so overlapping calls race); limit k * N <= 2^19 (N <= 16384 at an 868-bit q).
+        The plan's engine runs where its residues fit too, else the 62-bit one."""
         _check(load().nc_multiply_device_noalloc(self._h, _vp(d_a), _vp(d_b), _vp(d_c), _vp(stream or None)))
 
     def residues(self, d_x: int, d_r: int, engine: int = 0, stream: int = 0) -> None:
