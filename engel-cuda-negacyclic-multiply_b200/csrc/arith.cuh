@@ -19,9 +19,8 @@ __device__ __forceinline__ uint64_t csub(uint64_t x, uint64_t m) { return x >= m
 
 // Programmatic dependent launch. A product kernel launched with it may be scheduled while the
 // kernel before it on the stream still runs (once every CTA of that kernel has called
-// pdl_trigger(): on entry; in kernels that allocate tensor memory, once the CTA holds it; in the
-// 30-bit engine's kernels, after their own pdl_wait(), so that the CTAs of two products are never
-// resident at once), so its prologue (tensor-memory allocation, constant tables) overlaps that
+// pdl_trigger(): after its own pdl_wait() in the product kernels, so that the CTAs of two products
+// are never queued together, and once the CTA holds its tensor memory), so its prologue (tensor-memory allocation, constant tables) overlaps that
 // kernel's last wave.
 // pdl_wait() returns once the kernel before has completed and its writes are visible; every read
 // or write of data that kernel produces or consumes comes after it. In a kernel launched without

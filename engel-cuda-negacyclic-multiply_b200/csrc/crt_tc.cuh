@@ -170,6 +170,7 @@ __device__ void crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
     asm volatile("cp.async.commit_group;" ::: "memory");
     __syncthreads();
     pdl_wait();  // the residues come from the stream's previous kernel
+    pdl_trigger();
 
     switch (logN1) {
         case 0: crt_tc_detail::crt_columns_tc<0>(d, t, j0, T, s_y, s_ys, s_p, sA); break;

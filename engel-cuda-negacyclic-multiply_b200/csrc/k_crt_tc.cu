@@ -25,8 +25,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_crt_tc(ProductDesc d, Tables t)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // triggered only once the CTA holds its tensor memory (see k_dec_tc.cu)
-    pdl_trigger();
     const uint32_t taddr = taddr_slot;
     crt_coeffs_tc<LW>(d, t, int(blockIdx.x), smem, taddr, &bar, 0);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

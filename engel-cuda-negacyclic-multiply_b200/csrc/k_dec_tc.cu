@@ -110,14 +110,17 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
                      "l"(t.res_w), "r"(groups * 1024), "r"(smem_u32(&bars[1]))
                      : "memory");
     }
-    // The next kernel on the stream may be scheduled only once every CTA of this one holds its
-    // tensor memory: a dependent that allocates before its griddepcontrol.wait could otherwise
-    // take the columns a CTA of this kernel still waits for, and each would wait on the other.
     __syncthreads();
-    pdl_trigger();
 
     for (int w = tid; w < k; w += kThreads) s_p[w] = __ldg(t.primes + w);
     pdl_wait();  // the operand and the residue rows belong to the stream's previous kernels
+    // The next kernel may be scheduled only once every CTA of this one holds its tensor memory: a
+    // dependent that allocates before its griddepcontrol.wait could otherwise hold the columns this
+    // grid's CTAs need. And only after the wait, so that CTAs of two products never queue on the SMs
+    // together: triggered before it, kernels of N = 4096 stacked several CTAs on some SMs (three
+    // operands of 868 bits 98 us a product, 58 with the trigger here and in the row and CRT kernels;
+    // 1000 bits 58 and 50).
+    pdl_trigger();
     // A: 16-byte chunk q = (row group, K chunk, row), row m = u C + j is coefficient u N2 + j0 + j
     const int kbytes = 4 * L;
     for (int q = tid; q < kDecTcRows * 8; q += kThreads) {

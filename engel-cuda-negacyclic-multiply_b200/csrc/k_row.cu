@@ -10,7 +10,8 @@ namespace nc {
 template <int LOG_N2, int LOG_E, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 3 : 2) : 1)) k_row(ProductDesc d, Tables t) {
     extern __shared__ __align__(16) uint8_t smem[];
-    pdl_trigger();
+    pdl_wait();
+    pdl_trigger();  // after the wait, as k_dec_tc
     row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem);
 }
 

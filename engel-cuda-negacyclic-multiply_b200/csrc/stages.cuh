@@ -646,6 +646,7 @@ __device__ void crt_coeffs(const ProductDesc& d, const Tables& t, int tile, uint
     if (threadIdx.x < 4) s_mu[threadIdx.x] = __ldg(qc->mu + threadIdx.x);
     __syncthreads();  // s_p is read by the column stages
     pdl_wait();       // the residues come from the stream's previous kernel
+    pdl_trigger();
 
     switch (logN1) {
         case 0: crt_columns<0>(d, t, tile, s_p, s_res); break;
