@@ -182,6 +182,7 @@ int nc_plan_synchronize(nc_plan* plan) {
     return guarded([&] {
         if (!plan) throw nc::Error(nc::kEInval, "null plan");
         nc::check(cudaStreamSynchronize(plan->p->stream), "synchronize");
+        plan->p->tables->check_stuck();
     });
 }
 

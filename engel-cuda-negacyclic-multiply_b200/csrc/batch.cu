@@ -44,7 +44,7 @@ Batch::Batch(int device) : device_(device) {
     *err_host_ = 0;
 }
 
-bool Batch::failed() const { return ran_ && *err_host_ != 0; }
+bool Batch::failed() const { return ran_ && (*err_host_ != 0 || tables_->is_stuck()); }
 
 Batch::~Batch() {
     // wait on the batch's own event (never on the caller's stream, which may be gone)
@@ -473,6 +473,7 @@ void Batch::synchronize() {
 
 std::string Batch::failure() const {
     if (!failed()) return std::string();
+    if (*err_host_ == 0) return kStuck;
     return "a persistent-kernel dependency wait gave up (stage " + std::to_string(err_host_[1] >> 28) + ", product " +
            std::to_string(err_host_[1] & 0x0fffffffu) + ", saw " + std::to_string(err_host_[2]) + " of " +
            std::to_string(err_host_[3]) + ")";

@@ -52,9 +52,10 @@ class Batch {
         for (int c : n_dec_tc32_) n += c > 0 ? 1 : 0;
         return n;
     }
-    // After the last run has completed (its event): did a dependency wait give up?
+    // After the last run has completed (its event): did a dependency wait give up, or a kernel of the
+    // device report work that never completed (Tables::stuck)?
     bool failed() const;
-    // What the failed wait waited for (empty when nothing failed).
+    // What failed (empty when nothing did).
     std::string failure() const;
 
   private:

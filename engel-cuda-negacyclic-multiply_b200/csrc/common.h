@@ -178,7 +178,14 @@ struct Tables {
     const PrimeConst32* pc32;     // [kMaxPrimes32]
     const uint32_t* pow32_32;     // [kMaxPrimes32][kMaxL]: 2^(32 l) mod p_i
     const uint4* res_w32;         // [prime pairs][8 K chunks][8 rows: 4 byte planes of each][16 B]
+    // Host word that a kernel sets when a copy or MMA of its own is still in flight after two bounded
+    // waits (report_stuck, crt_tc.cuh): its results may then be wrong, and every later call on the device
+    // reports it.
+    uint32_t* stuck;
+    uint32_t give_up;             // tests: kGiveUp bits (NC_GIVE_UP when the tables are made), else 0
 };
+// First waits for copies give up at once; so do those for MMAs; second waits count as run out.
+enum : uint32_t { kGiveUpCopies = 1, kGiveUpMmas = 2, kGiveUpTwice = 4 };
 
 // Dynamic shared memory of each stage.
 NC_HD constexpr size_t smax(size_t a, size_t b) { return a > b ? a : b; }

@@ -39,8 +39,8 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ bool mma_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < kMmaWaitLimit; ++it) {
+__device__ __forceinline__ bool mma_wait(uint32_t bar, uint32_t parity, uint32_t polls = kMmaWaitLimit) {
+    for (uint32_t it = 0; it < polls; ++it) {
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -52,6 +52,20 @@ __device__ __forceinline__ bool mma_wait(uint32_t bar, uint32_t parity) {
         if (done) return true;
     }
     return false;
+}
+
+// Polls of the first wait for a copy.
+__device__ __forceinline__ uint32_t copy_polls(const Tables& t) { return t.give_up & kGiveUpCopies ? 0 : kMmaWaitLimit; }
+
+__device__ __forceinline__ void report_stuck(const Tables& t) {
+    *reinterpret_cast<volatile uint32_t*>(t.stuck) = 1;
+    __threadfence_system();
+}
+
+// One thread, once a first wait for phase `parity` of `bar` gave up and before the memory that the copy
+// writes is used for anything else or given back: waits again and reports if that runs out too.
+__device__ __forceinline__ void last_wait(const Tables& t, uint32_t bar, uint32_t parity) {
+    if (!mma_wait(bar, parity) || (t.give_up & kGiveUpTwice)) report_stuck(t);
 }
 
 // Byte offset of (row, byte) in an A half-tile: [16 row groups][16 K chunks][8 rows][16 B].

@@ -30,6 +30,10 @@ int current_device() {
 
 // ------------------------------------------------------------------------------ tables
 
+void DeviceTables::check_stuck() const {
+    if (is_stuck()) throw Error(kETimeout, kStuck);
+}
+
 namespace {
 std::mutex g_tables_mu;
 std::map<int, DeviceTables*> g_tables;
@@ -40,6 +44,7 @@ void free_tables(DeviceTables* t) {
                       static_cast<void*>(t->inv32), static_cast<void*>(t->pc32), static_cast<void*>(t->pow32_32),
                       static_cast<void*>(t->res_w32)})
         cudaFree(ptr);
+    cudaFreeHost(t->stuck);
 }
 
 // The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants, 2^(32 l) mod p,
@@ -91,6 +96,9 @@ DeviceTables* acquire_tables(int device) {
         check(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "device attribute");
         check(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device), "device attribute");
         t->tensor_cores = NC_HAS_TCGEN05 && major == 10 && minor == 0;
+        check(cudaHostAlloc(&t->stuck, 64, cudaHostAllocMapped | cudaHostAllocPortable), "status word");
+        *t->stuck = 0;
+        if (const char* g = std::getenv("NC_GIVE_UP")) t->give_up = uint32_t(std::atoi(g));
         const size_t tw_bytes = size_t(kMaxPrimes) * kMaxN * sizeof(ulonglong2);
         check(cudaMalloc(&t->fwd, tw_bytes), "twiddle table");
         check(cudaMalloc(&t->inv, tw_bytes), "inverse twiddle table");
@@ -564,6 +572,7 @@ void plan_multiply_device(Plan* p, const uint32_t* d_a, const uint32_t* d_b, uin
     if (((reinterpret_cast<uintptr_t>(d_a) | reinterpret_cast<uintptr_t>(d_b) | reinterpret_cast<uintptr_t>(d_c)) &
          15) != 0)
         throw Error(kEInval, "device buffers must be 16-byte aligned");
+    p->tables->check_stuck();
     ensure_scratch(p);
     const ProductDesc d = p->desc_plain(d_a, d_b, d_c);
     check(launch_product(d, p->tables->view(), p->plain_cfg(), stream, p->timing ? p->ev_stage : nullptr),
@@ -822,6 +831,7 @@ void plan_collect_host(Plan* p, uint32_t* c) {
         }
     });
     check(cudaError_t(err.load()), "product");
+    p->tables->check_stuck();
     // the last output chunk's event is the last work of the product on the plan's stream
     cudaEventElapsedTime(&p->last_kernel_ms, p->ev_start, p->ev_stop);
     if (p->trace) {
@@ -858,6 +868,7 @@ void plan_multiply_chain_device(Plan* p, const uint32_t* const* d_x, uint32_t* d
         align |= reinterpret_cast<uintptr_t>(d_x[f]);
     }
     if (align & 15) throw Error(kEInval, "device buffers must be 16-byte aligned");
+    p->tables->check_stuck();
     ensure_scratch(p);
     check(launch_product(p->desc_chain(d_x, d_c), p->tables->view(), p->cfg, stream,
                          p->timing ? p->ev_stage : nullptr),

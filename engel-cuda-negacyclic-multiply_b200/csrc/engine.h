@@ -28,6 +28,9 @@ enum : int { kOk = 0, kEInval = -1, kECuda = -2, kENoMem = -3, kETimeout = -4, k
 
 void check(cudaError_t e, const char* what);
 
+constexpr char kStuck[] =
+    "a kernel's copy or MMA did not complete within its bounded waits: products since then may be wrong";
+
 // Twiddles, residue places and prime constants for every prime of the set, resident on one
 // device (about 100 MB) while at least one plan on that device holds them.
 struct DeviceTables {
@@ -45,7 +48,15 @@ struct DeviceTables {
     PrimeConst32* pc32 = nullptr;
     uint32_t* pow32_32 = nullptr;
     uint4* res_w32 = nullptr;
-    Tables view() const { return Tables{fwd, inv, pow32, primes, res_w, fwd32, inv32, pc32, pow32_32, res_w32}; }
+    uint32_t* stuck = nullptr;  // pinned, written by the kernels (Tables::stuck)
+    uint32_t give_up = 0;
+    Tables view() const {
+        return Tables{fwd, inv, pow32, primes, res_w, fwd32, inv32, pc32, pow32_32, res_w32, stuck, give_up};
+    }
+    bool is_stuck() const { return stuck && *static_cast<volatile uint32_t*>(stuck) != 0; }
+    // Throws Error(kETimeout) once a kernel has reported work of its own that never completed. The word
+    // stays set: what such a copy overwrites, and when, is not known.
+    void check_stuck() const;
 };
 
 // Known answers of the host arithmetic, the prime set and sampled tables, checked once per

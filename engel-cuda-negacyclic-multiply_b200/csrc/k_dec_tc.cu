@@ -28,7 +28,9 @@ namespace nc {
 
 namespace {
 
+using crt_tc_detail::copy_polls;
 using crt_tc_detail::kmajor_desc;
+using crt_tc_detail::last_wait;
 using crt_tc_detail::mma_wait;
 using crt_tc_detail::smem_u32;
 
@@ -149,8 +151,12 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> MMA reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     // (the thread of the MMAs has also waited for the weights; if that gave up, the residues go by the
-    // integer pipes)
-    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0) ? 1 : 0) != 0;
+    // integer pipes, once the late copy has landed: they take its place)
+    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0, copy_polls(t)) ? 1 : 0) != 0;
+    if (failed) {
+        if (tid == 0) last_wait(t, smem_u32(&bars[1]), 0);
+        __syncthreads();
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     const int slices = (kbytes + 31) / 32;

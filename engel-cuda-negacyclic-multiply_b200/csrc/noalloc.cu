@@ -67,6 +67,7 @@ void multiply_noalloc(const Plan* p, const uint32_t* d_a, const uint32_t* d_b, u
     int device = -1;
     check(cudaGetDevice(&device), "cudaGetDevice");
     if (device != p->device) throw Error(kEInval, "the plan's device is not the current device");
+    p->tables->check_stuck();
     uint64_t* scratch = static_residues(device);
     const size_t words32 = (size_t(p->k32) * size_t(p->N) + 1) / 2;  // u64 words of one operand's u32 residues
     const bool w32 = p->use_w32() && 2 * words32 <= kStaticResidueWords;
