@@ -191,7 +191,8 @@ __device__ __forceinline__ void dec32_columns(uint32_t* R, const uint2* tw0, con
 // offsets are then constants), else 0. Primes [i0, i1), i0 a multiple of 32.
 template <int LOG_N1, int CC, int LN2>
 __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables& t, int operand, int tile, int i0,
-                                              int i1, uint8_t* smem, uint64_t (&bars)[2], uint32_t& taddr_slot) {
+                                              int i1, bool early, uint8_t* smem, uint64_t (&bars)[2],
+                                              uint32_t& taddr_slot) {
     uint64_t& bar = bars[0];
     const int N = 1 << d.logN;
     const int N2 = LN2 ? 1 << LN2 : N >> LOG_N1;
@@ -227,11 +228,13 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
         const PrimeConst32 pc = t.pc32[i0 + w];  // the MMAs' primes
         s_pc[w] = make_uint2(pc.p, pc.bar >> 2);
     }
+    if (early) pdl_trigger();
     pdl_wait();  // the operand and the residue rows belong to the stream's previous kernels
     // after the wait (and with the CTA's tensor memory in hand): the next kernel's CTAs are then placed
     // beside running CTAs, not beside a queue of waiting ones; at the kernel's entry, products of
     // N = 4096 to 16384 had kernels of two products resident at once, several row CTAs stacked on one
-    // SM (N = 8192, 868 bits: 28.7 us a product, 20.3 us with the trigger here)
+    // SM (N = 8192, 868 bits: 28.7 us a product, 20.3 us with the trigger here); where early_triggers
+    // says so, before the wait
     pdl_trigger();
     const int kbytes = 4 * L;
     for (int q = tid; q < kDecTcRows * 8; q += kThreads) {
@@ -351,13 +354,13 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
 // The item by its tile width and row length.
 template <int LOG_N1>
 __device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables& t, int operand, int tile, int i0, int i1,
-                                             uint8_t* smem, uint64_t (&bar)[2], uint32_t& taddr_slot) {
+                                             bool early, uint8_t* smem, uint64_t (&bar)[2], uint32_t& taddr_slot) {
     if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
-        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 12>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 12>(d, t, operand, tile, i0, i1, early, smem, bar, taddr_slot);
     else if (d.logN >= 7)
-        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 0>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+        dec_tc32_item<LOG_N1, (kDecTcRows >> LOG_N1), 0>(d, t, operand, tile, i0, i1, early, smem, bar, taddr_slot);
     else
-        dec_tc32_item<LOG_N1, 0, 0>(d, t, operand, tile, i0, i1, smem, bar, taddr_slot);
+        dec_tc32_item<LOG_N1, 0, 0>(d, t, operand, tile, i0, i1, early, smem, bar, taddr_slot);
 }
 
 // What bounds it: issue slots (the five-instruction fold of every residue, the column butterflies)
@@ -371,7 +374,7 @@ __device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables&
 // of its own).
 template <int LOG_N1>
 __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables t, int first_operand, int tile0,
-                                                           int tiles, int split) {
+                                                           int tiles, int split, int early) {
 #if NC_HAS_TCGEN05
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bar[2];
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
         if (i1 > i0 + kDecTc32PassPrimes) i1 = i0 + kDecTc32PassPrimes;
         b /= passes;
     }
-    dec_tc32_any<LOG_N1>(d, t, first_operand + b / tiles, tile0 + b % tiles, i0, i1, smem, bar, taddr_slot);
+    dec_tc32_any<LOG_N1>(d, t, first_operand + b / tiles, tile0 + b % tiles, i0, i1, early != 0, smem, bar, taddr_slot);
 #endif
 }
 
@@ -705,7 +708,7 @@ __device__ __forceinline__ void crt32_store(uint32_t* c, int N2, int L, int j0, 
 // two initialised mbarriers `bars` (the MMAs', the table's).
 template <int LOG_N1, int LN2>
 __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
-                                                uint8_t* smem, uint32_t taddr, uint64_t* bars) {
+                                                bool early, uint8_t* smem, uint32_t taddr, uint64_t* bars) {
     uint64_t* bar = bars;
     using A = Crt32Layout<LOG_N1>;
     // the descriptor's fields once (a batch's lies in global memory)
@@ -738,6 +741,7 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
     // issues them waits for it (its K bytes from 4 k up are zero, so A's are never read into the sums)
     if (tid == 0) bulk_table(sB, d.crt_b, uint32_t(NC) * 256u, smem_u32(bars + 1));
     __syncthreads();
+    if (early) pdl_trigger();
     pdl_wait();  // the residues come from the stream's previous kernel
     pdl_trigger();
 
@@ -806,7 +810,8 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
 
 // The tile within a kernel: tensor memory (`cols` columns) and the mbarrier around it.
 template <int LOG_N1>
-__device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t, int tile, int logT, uint32_t cols) {
+__device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t, int tile, int logT, uint32_t cols,
+                                          bool early) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bars[2];  // the MMAs', the table's
     __shared__ uint32_t taddr_slot;
@@ -826,9 +831,9 @@ __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t,
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
-        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, smem, taddr, bars);
+        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, early, smem, taddr, bars);
     else
-        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, smem, taddr, bars);
+        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, early, smem, taddr, bars);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32)
@@ -836,9 +841,10 @@ __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t,
 }
 
 template <int LOG_N1>
-__global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables t, int logT, uint32_t cols) {
+__global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables t, int logT, uint32_t cols,
+                                                           int early) {
 #if NC_HAS_TCGEN05
-    crt32_cta<LOG_N1>(d, t, int(blockIdx.x), logT, cols);
+    crt32_cta<LOG_N1>(d, t, int(blockIdx.x), logT, cols, early != 0);
 #endif
 }
 
@@ -851,9 +857,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables 
 // Resident CTAs per SM: radix-8 passes in 256-thread CTAs at four (64 registers: three and five CTAs
 // are no faster at N = 2^16), radix 16 at three.
 template <int LOG_N2, int LOG_E, int THREADS>
-__global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3) : 2)) k_row32(ProductDesc d, Tables t) {
+__global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3) : 2)) k_row32(ProductDesc d, Tables t,
+                                                                                                   int early) {
     extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint64_t bar;
+    if (early) pdl_trigger();
     const uint32_t b = smem_u32(&bar);
     w32::row_barrier_init<LOG_N2, LOG_E, THREADS>(b);
     w32::row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem, b, 0, true, true);
@@ -881,7 +889,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_dec_tc32(BatchCrtArgs a) 
     const BatchProduct& bp = a.products[w.x];
     const int tiles = int(bp.tiles_tc);
     const int operand = int(bp.first_operand) + int(w.y) / tiles, tile = int(w.y) % tiles;
-    dec_tc32_any<LOG_N1>(bp.d, a.tables, operand, tile, 0, int(bp.d.k), smem, bar, taddr_slot);
+    dec_tc32_any<LOG_N1>(bp.d, a.tables, operand, tile, 0, int(bp.d.k), false, smem, bar, taddr_slot);
 #endif
 }
 
@@ -955,7 +963,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_crt_tc32(BatchCrtArgs a, 
 #if NC_HAS_TCGEN05
     const uint2 w = __ldg(a.items + blockIdx.x);
     const ProductDesc& d = a.products[w.x].d;
-    crt32_cta<LOG_N1>(d, a.tables, int(w.y), crt32_batch_log_tile(int(d.logN)), cols);
+    crt32_cta<LOG_N1>(d, a.tables, int(w.y), crt32_batch_log_tile(int(d.logN)), cols, false);
 #endif
 }
 
@@ -1021,6 +1029,21 @@ void* batch_crt_tc32_kernel(int logN1) {
 }  // namespace
 
 }  // namespace w32
+
+// Which kernels of a plain product release the next one before their own wait (after it otherwise).
+// Early, the launch latencies of short kernels overlap; but the kernels of two products are then resident
+// at once and their CTAs placed unevenly, which costs more once kernels are longer. Early where that
+// measured faster (us a product, after the wait and early):
+// - up to N = 32, where a kernel has one CTA or few: N = 16, 31 bits 16.5 and 12.7, 868 bits 19.5 and
+//   17.1; N = 64, 434 bits 11.2 and 11.1, 600 bits at N = 128 11.3 and 11.7;
+// - rows and CRT from N = 2^14 up to 16 primes: at 2^14, 31 bits 18.1 and 15.0, 130 bits 19.2 and 17.1;
+//   at 2^16, 31 bits 21.8 and 20.7; but 200 bits at 2^13 12.9 and 14.0, 300 bits (21 primes) at 2^15
+//   21.9 and 22.5.
+enum : int { kEarlyDec = 1, kEarlyRow = 2, kEarlyCrt = 4 };
+static int early_triggers(int logN, int k) {
+    if (logN <= 5) return kEarlyDec | kEarlyRow | kEarlyCrt;
+    return logN >= 14 && k <= 16 ? kEarlyRow | kEarlyCrt : 0;
+}
 
 // Residue launches of at most this many CTAs give each pass of primes its own CTA.
 constexpr int kDec32SplitCtas = 74;
@@ -1117,7 +1140,8 @@ cudaError_t launch_residues32(const ProductDesc& d, const Tables& t, int logN1, 
     const int passes = (int(d.k) + kDecTc32PassPrimes - 1) / kDecTc32PassPrimes;
     int split = count * tiles * passes <= kDec32SplitCtas ? 1 : 0;
     const int primes = split && int(d.k) > kDecTc32PassPrimes ? kDecTc32PassPrimes : int(d.k);
-    void* args[] = {&dd, &tt, &first, &tile0, &tiles, &split};
+    int early = early_triggers(int(d.logN), int(d.k)) & kEarlyDec;
+    void* args[] = {&dd, &tt, &first, &tile0, &tiles, &split, &early};
     return launch_pdl(fn, count * tiles * (split ? passes : 1), kThreads, dec_tc32_smem_bytes(primes), s, args);
 }
 
@@ -1127,7 +1151,8 @@ cudaError_t launch_row32(const ProductDesc& d, const Tables& t, const RowConfig&
     const Geometry g = geometry(int(d.logN), int(d.k), cfg);
     ProductDesc dd = d;
     Tables tt = t;
-    void* args[] = {&dd, &tt};
+    int early = early_triggers(int(d.logN), int(d.k)) & kEarlyRow;
+    void* args[] = {&dd, &tt, &early};
     return launch_pdl(fn, g.row_ctas, cfg.threads, w32::row_smem_bytes(cfg.threads, cfg.logE), s, args);
 }
 
@@ -1139,7 +1164,8 @@ cudaError_t launch_crt32(const ProductDesc& d, const Tables& t, cudaStream_t s) 
     Tables tt = t;
     int logT = crt32_log_tile(int(d.logN), logN1);
     uint32_t cols = crt32_tmem_cols(int(d.LW));
-    void* args[] = {&dd, &tt, &logT, &cols};
+    int early = early_triggers(int(d.logN), int(d.k)) & kEarlyCrt;
+    void* args[] = {&dd, &tt, &logT, &cols, &early};
     return launch_pdl(fn, 1 << (int(d.logN) - logT), kThreads, w32::crt_tc32_smem_bytes(int(d.LW)), s, args);
 }
 
