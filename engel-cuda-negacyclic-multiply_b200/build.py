@@ -5,6 +5,8 @@
 
 Outputs (git-ignored, shipped with the tree):
     lib/libnegacyclic_b200.so   C ABI (include/negacyclic_b200.h) + fherma_init/run/free
+    lib/libnegacyclic_b200_give_up.so
+                                the same for tests: kernels' waits can be made to run out
     bin/solution                harness runner: reads a case directory, writes out/*/c.bin
     dropin/solve.cu             the whole library as one source file, for a platform project that
                                 accepts solve.cu and nothing else (its generated CMakeLists.txt
@@ -26,6 +28,7 @@ CSRC = PKG / "csrc"
 INCLUDE = ROOT / "include"
 OBJ = PKG / "_build"
 LIB = PKG / "lib" / "libnegacyclic_b200.so"
+GIVE_UP_LIB = PKG / "lib" / "libnegacyclic_b200_give_up.so"
 BIN = PKG / "bin" / "solution"
 SOLVE_CU = PKG / "dropin" / "solve.cu"
 
@@ -36,6 +39,9 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", f"-I{INCLUDE}
 LIB_SOURCES = ["hostmath.cpp", "k_dec.cu", "k_row.cu", "k_crt.cu", "k_batch.cu", "kernels.cu", "batch.cu",
                "engine.cu", "server.cu", "api.cu", "noalloc.cu", "k_residues.cu", "k_crt_tc.cu", "k_dec_tc.cu",
                "k_w32.cu"]
+# Sources of the library whose code depends on NC_TEST_GIVE_UP: the kernels that wait on a copy or on
+# MMAs, and the plan's side of it.
+GIVE_UP_SOURCES = ["k_batch.cu", "engine.cu", "k_crt_tc.cu", "k_dec_tc.cu", "k_w32.cu"]
 RUNNER_SOURCES = ["runner.cpp"]
 
 
@@ -67,17 +73,19 @@ def _stale(target: Path, deps: list[Path]) -> bool:
     return any(d.stat().st_mtime > t for d in deps)
 
 
-def _compile(src: Path, verbose: bool) -> Path:
-    obj = OBJ / (src.name + ".o")
+def _compile(src: Path, verbose: bool, give_up: bool = False) -> Path:
+    obj = OBJ / (src.name + (".give_up.o" if give_up else ".o"))
     if not _stale(obj, [src] + _headers(src)):
         return obj
     cmd = [NVCC, *ARCH, *COMMON, "-c", str(src), "-o", str(obj)]
-    if src.suffix == ".cu" and verbose:
+    if give_up:
+        cmd.insert(1, "-DNC_TEST_GIVE_UP")
+    elif src.suffix == ".cu" and verbose:
         cmd.insert(1, "-Xptxas=-v")
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"compile failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
-    if verbose and r.stderr:
+    if verbose and r.stderr and not give_up:
         (OBJ / (src.name + ".ptxas.txt")).write_text(r.stderr)
     return obj
 
@@ -157,12 +165,15 @@ def build(clean: bool = False, verbose: bool = False) -> Path:
     BIN.parent.mkdir(parents=True, exist_ok=True)
     sources = [CSRC / s for s in LIB_SOURCES if (CSRC / s).exists()]
     with cf.ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1))) as ex:
-        objs = list(ex.map(lambda s: _compile(s, verbose), sources))
-    if _stale(LIB, objs):
-        cmd = [NVCC, *ARCH, "-shared", "-o", str(LIB), *map(str, objs), "-lpthread"]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        if r.returncode != 0:
-            raise RuntimeError(f"link failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+        todo = [(s, False) for s in sources] + [(CSRC / s, True) for s in GIVE_UP_SOURCES]
+        done = dict(zip(todo, ex.map(lambda t: _compile(t[0], verbose, t[1]), todo)))
+    objs = [done[s, False] for s in sources]
+    for lib, parts in ((LIB, objs), (GIVE_UP_LIB, [done.get((s, True), done[s, False]) for s in sources])):
+        if _stale(lib, parts):
+            cmd = [NVCC, *ARCH, "-shared", "-o", str(lib), *map(str, parts), "-lpthread"]
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"link failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
     runner = [CSRC / s for s in RUNNER_SOURCES if (CSRC / s).exists()]
     if runner and _stale(BIN, runner + [LIB] + _headers()):
         cmd = ["g++", "-O2", "-std=c++17", f"-I{INCLUDE}", *map(str, runner), "-o", str(BIN),

@@ -17,6 +17,32 @@ constexpr uint64_t kMask62 = (1ull << 62) - 1;
 
 __device__ __forceinline__ uint64_t csub(uint64_t x, uint64_t m) { return x >= m ? x - m : x; }
 
+// Waits for phase `parity` of the mbarrier at shared address `bar`, which a copy or MMAs (`what`) complete:
+// false if they have not within the limit.
+__device__ __forceinline__ bool bar_wait(const Tables& t, uint32_t bar, uint32_t parity, uint32_t what) {
+    for (uint32_t it = 0; it < (1u << 23); ++it) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+#ifdef NC_TEST_GIVE_UP
+        if (done && (reinterpret_cast<uintptr_t>(t.stuck) & what)) return false;
+#endif
+        if (done) return true;
+    }
+    return false;
+}
+
+// A CTA whose wait ran out tells the host, frees its tensor memory and ends without a result: what still
+// writes its memory, and when, is not known.
+__device__ __forceinline__ void report_stuck(const Tables& t) {
+    *reinterpret_cast<volatile uint32_t*>(reinterpret_cast<uintptr_t>(t.stuck) & ~uintptr_t(kGiveUpBits)) = 1;
+}
+
 // Programmatic dependent launch. A product kernel launched with it may be scheduled while the
 // kernel before it on the stream still runs (once every CTA of that kernel has called
 // pdl_trigger(): after its own pdl_wait() in the product kernels, so that the CTAs of two products

@@ -111,16 +111,15 @@ constexpr int kDecTc32PassPrimes = 32;   // residue MMAs: 4 byte planes x 32 pri
 struct PrimeConst32 {
     uint32_t p;
     uint32_t pinv;  // -p^-1 mod 2^32 (Montgomery)
-    uint32_t bar;   // floor(2^50 / p): reduction of a 48-bit folded residue sum
-    uint32_t quo;   // floor(2^61 / p): the CRT quotient estimate
+    uint32_t c48;   // floor(2^48 / p): reduction of a residue's byte-plane sums (fold_planes)
+    uint32_t pad;
 };
 
-// Per-(q, N) constants of the 30-bit engine's CRT + Barrett stage.
+// Per-(q, N) constants of the 30-bit engine's CRT stage.
 struct QConst32 {
     uint32_t L, LW, k, qbits, logN, pad0;
     uint32_t q[kMaxL + 2];
     uint32_t neg_m[kMaxL + 2];             // (-M) mod q, M = prod of the k primes
-    uint32_t mu[4];                        // floor(2^(qbits + kBarrettT + 1) / q)
     // one-word quotient of the tensor-core CRT (crt32_finish in k_w32.cu): a sum T < 2^17 q has
     // floor(T / q) = umulhi(floor(T / 2^(qbits - 14)), mu1) >> 13, or one less
     uint32_t top_byte;                     // c0 = max(0, floor((qbits - 1) / 8) - 4): bytes c0 .. c0 + 4 of T
@@ -130,7 +129,6 @@ struct QConst32 {
     uint64_t top_neg_m;                    // floor(((-M) mod q) / 2^(8 c0))
     uint32_t neg_q[kMaxL + 2];             // 2^(32 (LW + 1)) - q
     uint32_t y[kMaxPrimes32];              // (M/p_i)^-1 N^-1 2^32 mod p_i (2^32: the pointwise Montgomery factor)
-    uint32_t ys[kMaxPrimes32];             // floor(y 2^32 / p_i)
     uint32_t mq[kMaxPrimes32 * (kMaxL + 2)];  // (M/p_i) mod q, row stride kMaxL + 2
 };
 
@@ -176,16 +174,14 @@ struct Tables {
     const uint2* fwd32;           // [kMaxPrimes32][kMaxN]: psi^bitrev16(j) and floor(w 2^32 / p)
     const uint2* inv32;           // [kMaxPrimes32][kMaxN]: psi^-bitrev16(j) and its companion
     const PrimeConst32* pc32;     // [kMaxPrimes32]
-    const uint32_t* pow32_32;     // [kMaxPrimes32][kMaxL]: 2^(32 l) mod p_i
     const uint4* res_w32;         // [prime pairs][8 K chunks][8 rows: 4 byte planes of each][16 B]
-    // Host word that a kernel sets when a copy or MMA of its own is still in flight after two bounded
-    // waits (report_stuck, crt_tc.cuh): its results may then be wrong, and every later call on the device
-    // reports it.
+    // Host word that a kernel sets when a copy or MMAs of its own have not completed within their bounded
+    // wait (bar_wait): its CTA ends without a result, and every later call on the device reports it. In test
+    // builds the word's address carries kGiveUp bits.
     uint32_t* stuck;
-    uint32_t give_up;             // tests: kGiveUp bits (NC_GIVE_UP when the tables are made), else 0
 };
-// First waits for copies give up at once; so do those for MMAs; second waits count as run out.
-enum : uint32_t { kGiveUpCopies = 1, kGiveUpMmas = 2, kGiveUpTwice = 4 };
+// NC_TEST_GIVE_UP builds: waits for copies, and waits for MMAs, that count as run out once they are over.
+enum : uint32_t { kGiveUpCopies = 1, kGiveUpMmas = 2, kGiveUpBits = 3 };
 
 // Dynamic shared memory of each stage.
 NC_HD constexpr size_t smax(size_t a, size_t b) { return a > b ? a : b; }

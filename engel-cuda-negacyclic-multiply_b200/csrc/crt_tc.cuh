@@ -14,8 +14,7 @@
 // integer-pipe kernel forms. The tile's 256 coefficients are two M = 128 MMAs per 32-byte K slice
 // (tcgen05.mma.cta_group::1.kind::i8), accumulators in tensor memory; each thread then folds its
 // row of S into 32-bit words with one carry pass, adds K (-M mod q) and runs the Barrett reduction
-// of crt_coeffs. If the bounded wait for the MMAs gives up, the thread forms the sum with the
-// integer carry chains instead, so the result never depends on the wait.
+// of crt_coeffs.
 #pragma once
 
 #include "stages.cuh"
@@ -33,39 +32,8 @@ __device__ __forceinline__ uint64_t kmajor_desc(uint32_t addr, uint32_t lbo, uin
            (uint64_t((sbo >> 4) & 0x3FFFu) << 32) | (uint64_t(1) << 46);
 }
 
-constexpr uint32_t kMmaWaitLimit = 1u << 22;
-
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-
-__device__ __forceinline__ bool mma_wait(uint32_t bar, uint32_t parity, uint32_t polls = kMmaWaitLimit) {
-    for (uint32_t it = 0; it < polls; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-// Polls of the first wait for a copy.
-__device__ __forceinline__ uint32_t copy_polls(const Tables& t) { return t.give_up & kGiveUpCopies ? 0 : kMmaWaitLimit; }
-
-__device__ __forceinline__ void report_stuck(const Tables& t) {
-    *reinterpret_cast<volatile uint32_t*>(t.stuck) = 1;
-    __threadfence_system();
-}
-
-// One thread, once a first wait for phase `parity` of `bar` gave up and before the memory that the copy
-// writes is used for anything else or given back: waits again and reports if that runs out too.
-__device__ __forceinline__ void last_wait(const Tables& t, uint32_t bar, uint32_t parity) {
-    if (!mma_wait(bar, parity) || (t.give_up & kGiveUpTwice)) report_stuck(t);
 }
 
 // Byte offset of (row, byte) in an A half-tile: [16 row groups][16 K chunks][8 rows][16 B].
@@ -142,9 +110,9 @@ __device__ void crt_columns_tc(const ProductDesc& d, const Tables& t, int j0, in
 
 // One 256-coefficient tile (index `tile`) with every thread of a 256-thread CTA. The caller owns
 // crt_tc_tmem_cols(LW) columns of tensor memory at `taddr` and an initialised mbarrier `bar`
-// whose phase `parity` the MMAs of this call complete.
+// whose phase `parity` the MMAs of this call complete; false if they did not in time.
 template <int LW>
-__device__ void crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, uint8_t* smem, uint32_t taddr,
+__device__ bool crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, uint8_t* smem, uint32_t taddr,
                               uint64_t* bar, uint32_t parity) {
     constexpr int W = LW + kAccExtra;
     constexpr int NC = crt_tc_cols(LW);
@@ -234,12 +202,13 @@ __device__ void crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
     }
     const uint32_t kq = uint32_t((frac + (1ull << 31)) >> 32);
 
-    const bool ok = crt_tc_detail::mma_wait(crt_tc_detail::smem_u32(bar), parity);
+    // one warp polls, the others wait at the barrier
+    if (!__syncthreads_and(warp != 0 || bar_wait(t, crt_tc_detail::smem_u32(bar), parity, kGiveUpMmas) ? 1 : 0)) return false;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t acc[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) acc[w] = 0;
-    if (__all_sync(0xffffffffu, ok)) {
+    {
         // fold S_c 2^(8c) into 32-bit words: two words per group of eight columns, one carry pass
         const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(half) * kHalfCol;
         uint64_t carry = 0;
@@ -258,27 +227,6 @@ __device__ void crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
             if (2 * cb + 1 < W) acc[2 * cb + 1] = uint32_t(t1);
             carry = t1 >> 32;
         }
-    } else {
-        // the MMAs did not report completion in time: the same sum on the integer pipes
-        uint32_t acc_hi[W];
-#pragma unroll
-        for (int w = 0; w < W; ++w) acc_hi[w] = 0;
-#pragma unroll 1
-        for (int i = 0; i < k; ++i) {
-            const uint64_t v = *reinterpret_cast<const uint64_t*>(arow + (i >> 1) * 128 + (i & 1) * 8);
-            const uint32_t* M = qc->mq + i * kMqStride;
-            uint32_t m[LW];
-#pragma unroll
-            for (int l = 0; l < LW; ++l) m[l] = __ldg(M + l);
-            mac_lo<LW, 0, W>(acc, m, uint32_t(v));
-            mac_hi<LW, 1, W>(acc_hi, m, uint32_t(v));
-            mac_lo<LW, 1, W>(acc, m, uint32_t(v >> 32));
-            mac_hi<LW, 2, W>(acc_hi, m, uint32_t(v >> 32));
-        }
-        asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(acc_hi[0]));
-#pragma unroll
-        for (int w = 1; w < W - 1; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[w]) : "r"(acc_hi[w]));
-        asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[W - 1]) : "r"(acc_hi[W - 1]));
     }
     // acc += round(sum v_i / p_i) * ((-M) mod q)
     {
@@ -317,6 +265,7 @@ __device__ void crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
     }
     __syncthreads();
     store_tile(d.c, N2, L, j0, C, 1 << logN1, s_out);
+    return true;
 }
 
 }  // namespace nc

@@ -30,6 +30,14 @@ int current_device() {
 
 // ------------------------------------------------------------------------------ tables
 
+Tables DeviceTables::view() const {
+    uintptr_t word = reinterpret_cast<uintptr_t>(stuck);
+#ifdef NC_TEST_GIVE_UP
+    if (const char* g = std::getenv("NC_GIVE_UP")) word |= uintptr_t(std::atoi(g)) & kGiveUpBits;
+#endif
+    return Tables{fwd, inv, pow32, primes, res_w, fwd32, inv32, pc32, res_w32, reinterpret_cast<uint32_t*>(word)};
+}
+
 void DeviceTables::check_stuck() const {
     if (is_stuck()) throw Error(kETimeout, kStuck);
 }
@@ -41,14 +49,12 @@ std::map<int, DeviceTables*> g_tables;
 void free_tables(DeviceTables* t) {
     for (void* ptr : {static_cast<void*>(t->fwd), static_cast<void*>(t->inv), static_cast<void*>(t->pow32),
                       static_cast<void*>(t->primes), static_cast<void*>(t->res_w), static_cast<void*>(t->fwd32),
-                      static_cast<void*>(t->inv32), static_cast<void*>(t->pc32), static_cast<void*>(t->pow32_32),
-                      static_cast<void*>(t->res_w32)})
+                      static_cast<void*>(t->inv32), static_cast<void*>(t->pc32), static_cast<void*>(t->res_w32)})
         cudaFree(ptr);
     cudaFreeHost(t->stuck);
 }
 
-// The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants, 2^(32 l) mod p,
-// and the residue stage's weight bytes (byte c of 2^(8 b) mod p_i at
+// The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants and the residue stage's weight bytes (byte c of 2^(8 b) mod p_i at
 // [i / 2][b / 16][4 (i % 2) + c][b % 16], b < 128: the MMA's B rows of a prime pair).
 void upload_tables32(DeviceTables* t) {
     const HostTables32& h = host_tables32();
@@ -60,9 +66,6 @@ void upload_tables32(DeviceTables* t) {
     check(cudaMalloc(&t->pc32, size_t(kMaxPrimes32) * sizeof(PrimeConst32)), "30-bit prime table");
     check(cudaMemcpy(t->pc32, h.pc.data(), size_t(kMaxPrimes32) * sizeof(PrimeConst32), cudaMemcpyHostToDevice),
           "30-bit prime upload");
-    check(cudaMalloc(&t->pow32_32, size_t(kMaxPrimes32) * kMaxL * 4), "30-bit limb weights");
-    check(cudaMemcpy(t->pow32_32, h.pow32.data(), size_t(kMaxPrimes32) * kMaxL * 4, cudaMemcpyHostToDevice),
-          "30-bit limb weight upload");
     std::vector<uint8_t> w(size_t(kMaxPrimes32 / 2) * 1024, 0);
     for (int i = 0; i < kMaxPrimes32; ++i) {
         const uint64_t p = h.pc[size_t(i)].p;
@@ -98,7 +101,6 @@ DeviceTables* acquire_tables(int device) {
         t->tensor_cores = NC_HAS_TCGEN05 && major == 10 && minor == 0;
         check(cudaHostAlloc(&t->stuck, 64, cudaHostAllocMapped | cudaHostAllocPortable), "status word");
         *t->stuck = 0;
-        if (const char* g = std::getenv("NC_GIVE_UP")) t->give_up = uint32_t(std::atoi(g));
         const size_t tw_bytes = size_t(kMaxPrimes) * kMaxN * sizeof(ulonglong2);
         check(cudaMalloc(&t->fwd, tw_bytes), "twiddle table");
         check(cudaMalloc(&t->inv, tw_bytes), "inverse twiddle table");

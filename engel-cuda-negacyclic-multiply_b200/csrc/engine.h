@@ -46,13 +46,9 @@ struct DeviceTables {
     uint2* fwd32 = nullptr;
     uint2* inv32 = nullptr;
     PrimeConst32* pc32 = nullptr;
-    uint32_t* pow32_32 = nullptr;
     uint4* res_w32 = nullptr;
     uint32_t* stuck = nullptr;  // pinned, written by the kernels (Tables::stuck)
-    uint32_t give_up = 0;
-    Tables view() const {
-        return Tables{fwd, inv, pow32, primes, res_w, fwd32, inv32, pc32, pow32_32, res_w32, stuck, give_up};
-    }
+    Tables view() const;
     bool is_stuck() const { return stuck && *static_cast<volatile uint32_t*>(stuck) != 0; }
     // Throws Error(kETimeout) once a kernel has reported work of its own that never completed. The word
     // stays set: what such a copy overwrites, and when, is not known.

@@ -522,8 +522,7 @@ std::vector<PrimeConst32> make_prime_set32() {
         PrimeConst32 c{};
         c.p = uint32_t(cand);
         c.pinv = 0u - inv;
-        c.bar = uint32_t((1ull << 50) / cand);
-        c.quo = uint32_t((1ull << 61) / cand);
+        c.c48 = uint32_t((1ull << 48) / cand);
         out.push_back(c);
     }
     return out;
@@ -555,7 +554,6 @@ const HostTables32& host_tables32() {
     std::call_once(once, [] {
         t.pc = prime_set32();
         t.psi.assign(kMaxPrimes32, 0);
-        t.pow32.assign(size_t(kMaxPrimes32) * kMaxL, 0);
         t.fwd.assign(size_t(kMaxPrimes32) * kMaxN * 2, 0);
         t.inv.assign(size_t(kMaxPrimes32) * kMaxN * 2, 0);
         auto work = [](int i) {
@@ -569,11 +567,6 @@ const HostTables32& host_tables32() {
                 }
             }
             t.psi[size_t(i)] = uint32_t(psi);
-            uint64_t place = 1;
-            for (int l = 0; l < kMaxL; ++l) {
-                t.pow32[size_t(i) * kMaxL + size_t(l)] = uint32_t(place);
-                place = (place << 32) % p;
-            }
             std::vector<uint32_t> pw(kMaxN + 1);
             pw[0] = 1;
             for (int e = 1; e <= kMaxN; ++e) pw[size_t(e)] = uint32_t(uint64_t(pw[size_t(e) - 1]) * psi % p);
@@ -610,8 +603,7 @@ std::string check_prime_set32() {
         if (((c.p - 1) & ((1u << kRootLog) - 1)) != 0) return at + "not 1 mod 2^17";
         if (c.p >= (1u << 30) || c.p <= (1u << 29)) return at + "not in (2^29, 2^30)";
         if (uint32_t(c.p * (0u - c.pinv)) != 1u) return at + "pinv is not -p^-1 mod 2^32";
-        if (uint64_t(c.bar) != (1ull << 50) / c.p || uint64_t(c.quo) != (1ull << 61) / c.p)
-            return at + "reciprocal constants";
+        if (uint64_t(c.c48) != (1ull << 48) / c.p) return at + "reciprocal constant";
         if (i > 0 && c.p >= ps[size_t(i) - 1].p) return "30-bit prime set not descending";
     }
     return std::string();
@@ -623,9 +615,6 @@ std::string check_tables32(const HostTables32& t, int samples) {
         const uint64_t psi = t.psi[size_t(i)];
         const std::string at = "30-bit prime " + std::to_string(i) + ": ";
         if (powmod64(psi, 1ull << kMaxLogN, p) != p - 1) return at + "psi^(2^16) != -1";
-        for (int l = 0; l < kMaxL; ++l)
-            if (t.pow32[size_t(i) * kMaxL + size_t(l)] != powmod64(2, 32ull * uint64_t(l), p))
-                return at + "2^(32 l) mod p";
         const uint32_t* f = t.fwd.data() + size_t(i) * kMaxN * 2;
         const uint32_t* g = t.inv.data() + size_t(i) * kMaxN * 2;
         for (int s = 0; s < samples; ++s) {
@@ -672,7 +661,6 @@ std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out) {
         const uint64_t y = mulmod64(mulmod64(powmod64(mi_mod_p, p - 2, p), powmod64(N % p, p - 2, p), p),
                                     (1ull << 32) % p, p);
         out->y[i] = uint32_t(y);
-        out->ys[i] = shoup32(uint32_t(y), uint32_t(p));
         const Big miq = divmod(Mi, qb, nullptr);
         for (size_t l = 0; l < miq.size() && l < size_t(kMqStride); ++l) out->mq[size_t(i) * kMqStride + l] = miq[l];
     }
@@ -682,10 +670,6 @@ std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out) {
     else neg.clear();
     if (cmp_big(neg, qb) == 0) neg.clear();
     for (size_t l = 0; l < neg.size(); ++l) out->neg_m[l] = neg[l];
-    Big mu;
-    divmod(pow2(qbits + kBarrettT + 1), qb, &mu);
-    if (bits_of(mu) > 96) return "internal: Barrett constant too wide";
-    for (size_t l = 0; l < mu.size() && l < 4; ++l) out->mu[l] = mu[l];
     const int c0 = std::max(0, (qbits - 1) / 8 - 4);
     out->top_byte = uint32_t(c0);
     out->top_shift = qbits - 8 * c0 - 14;
@@ -750,17 +734,12 @@ std::string check_qconst32(const QConst32& c) {
             if (j != i) mi = mulmod64(mi, ps[size_t(j)].p % p, p);
         // y_i (M / p_i) N = 2^32 (mod p_i)
         if (mulmod64(mulmod64(c.y[i], mi, p), N % p, p) != (1ull << 32) % p) return at + "y_i (M/p_i) N != 2^32";
-        const uint64_t lhs = uint64_t(c.y[i]) << 32, qp = uint64_t(c.ys[i]) * p;
-        if (c.y[i] >= p || qp > lhs || lhs - qp >= p) return at + "Shoup companion of y_i";
+        if (c.y[i] >= p) return at + "y_i is not below p_i";
         Big mq(c.mq + size_t(i) * kMqStride, c.mq + size_t(i) * kMqStride + kMqStride);
         trim(mq);
         if (cmp_big(mq, qb) >= 0) return at + "(M/p_i) mod q is not below q";
         if (!divmod(add_big(mul_u64(mq, p), neg), qb, nullptr).empty()) return at + "(M/p_i mod q) p_i != M mod q";
     }
-    Big mu(c.mu, c.mu + 4);
-    trim(mu);
-    const Big e = pow2(int(c.qbits) + kBarrettT + 1);
-    if (cmp_big(mul_big(mu, qb), e) > 0 || cmp_big(add_big(mul_big(mu, qb), qb), e) <= 0) return "Barrett constant mu";
     Big m1{c.mu1};
     const Big e1 = pow2(int(c.qbits) + 31);
     if (bits_of(qb) > 1 && (cmp_big(mul_big(m1, qb), e1) > 0 || cmp_big(add_big(mul_big(m1, qb), qb), e1) <= 0))

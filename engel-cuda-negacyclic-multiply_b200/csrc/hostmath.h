@@ -50,7 +50,6 @@ std::string check_qconst(const QConst& c);                   // CRT identities a
 struct HostTables32 {
     std::vector<PrimeConst32> pc;  // kMaxPrimes32, descending below 2^30
     std::vector<uint32_t> psi;     // primitive 2^17-th root of unity per prime
-    std::vector<uint32_t> pow32;   // kMaxPrimes32 * kMaxL: 2^(32 l) mod p
     std::vector<uint32_t> fwd;     // kMaxPrimes32 * kMaxN * 2 (w, floor(w 2^32 / p))
     std::vector<uint32_t> inv;     // same for psi^-1
 };
@@ -72,7 +71,7 @@ std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out);
 std::vector<uint8_t> crt32_table(const QConst32& c);
 
 std::string check_prime_set32();                                 // primes, 1 mod 2^17, constants
-std::string check_tables32(const HostTables32& t, int samples);  // psi, 2^(32 l) mod p, twiddles
+std::string check_tables32(const HostTables32& t, int samples);  // psi, sampled twiddles
 std::string check_qconst32(const QConst32& c);                   // CRT identities and mu
 
 // c = a * b mod (X^N + 1, q) by the schoolbook sum on big integers (small N only: the device

@@ -192,16 +192,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_batch_crt_tc(BatchCrtArgs a) {
     const uint32_t taddr = taddr_slot;
     const uint2 w = __ldg(a.items + blockIdx.x);
     const BatchProduct& bp = a.products[w.x];
+    bool ok = true;
     switch (bp.d.LW) {
-#define NC_B_CRT_TC(n)                                                        \
-    case n:                                                                   \
-        if constexpr (crt_tc_tmem_cols(n) == 256)                             \
-            crt_coeffs_tc<n>(bp.d, a.tables, int(w.y), smem, taddr, &bar, 0); \
+#define NC_B_CRT_TC(n)                                                             \
+    case n:                                                                        \
+        if constexpr (crt_tc_tmem_cols(n) == 256)                                  \
+            ok = crt_coeffs_tc<n>(bp.d, a.tables, int(w.y), smem, taddr, &bar, 0); \
         break;
         NC_LW_CASES(NC_B_CRT_TC)
 #undef NC_B_CRT_TC
         default: break;
     }
+    if (!ok) report_stuck(a.tables);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(taddr) : "memory");

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_crt_tc(ProductDesc d, Tables t)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
-    crt_coeffs_tc<LW>(d, t, int(blockIdx.x), smem, taddr, &bar, 0);
+    if (!crt_coeffs_tc<LW>(d, t, int(blockIdx.x), smem, taddr, &bar, 0)) report_stuck(t);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32)

@@ -11,15 +11,14 @@
 // x 128 K bytes (4 L, zero padded) x 8 columns per prime, every S < 128 * 255^2 < 2^23, so the s32
 // accumulation in tensor memory is exact. The primes (any count up to 48) go through
 // tcgen05.mma kind::i8 in passes of 16 (128 accumulator columns); after each pass the eight warps
-// read the partial sums back
-// (tcgen05.ld) and fold sum_c 2^(8 c) S_c (< 2^80) into [0, 2p) modulo p_i. The tile is
+// read the partial sums back (tcgen05.ld) and fold sum_c 2^(8 c) S_c (< 2^80) into [0, 2p) modulo p_i.
+// The tile is
 // C = 128 / N1 columns of all N1 rows of the polynomial (row length N2 = N / N1), as in k_dec, so
 // the forward column stages and the residue-row stores follow unchanged.
 //
-// Operand and weight bytes reach shared memory by cp.async (no register staging). Each prime's
-// residues overwrite its own 1 KB of weights once its pass's MMAs have completed. If the bounded
-// wait for a pass gives up, each warp forms its
-// residues with the integer carry chains of k_dec instead, so the result never depends on it.
+// Operand bytes reach shared memory by cp.async, the weights by one bulk copy (no register staging).
+// Each prime's residues overwrite its own 1 KB of weights once its pass's MMAs have completed. A bounded
+// wait that runs out ends the CTA without a result and is reported (report_stuck).
 #include "batch_types.h"
 #include "crt_tc.cuh"
 #include "kernel_registry.h"
@@ -28,10 +27,7 @@ namespace nc {
 
 namespace {
 
-using crt_tc_detail::copy_polls;
 using crt_tc_detail::kmajor_desc;
-using crt_tc_detail::last_wait;
-using crt_tc_detail::mma_wait;
 using crt_tc_detail::smem_u32;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -150,13 +146,8 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> MMA reads
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // (the thread of the MMAs has also waited for the weights; if that gave up, the residues go by the
-    // integer pipes, once the late copy has landed: they take its place)
-    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0, copy_polls(t)) ? 1 : 0) != 0;
-    if (failed) {
-        if (tid == 0) last_wait(t, smem_u32(&bars[1]), 0);
-        __syncthreads();
-    }
+    // (the thread of the MMAs has also waited for the weights)
+    bool ok = __syncthreads_and(tid != 0 || bar_wait(t, smem_u32(&bars[1]), 0, kGiveUpCopies) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     const int slices = (kbytes + 31) / 32;
@@ -165,10 +156,10 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     // and half w / 4 of the pass's primes
     const int m = 32 * (warp & 3) + lane;
     const int half = warp >> 2;
-    for (int g = 0; g * kDecTcPassPrimes < k; ++g) {
+    for (int g = 0; ok && g * kDecTcPassPrimes < k; ++g) {
         const int i0 = g * kDecTcPassPrimes;
         const int np = k - i0 < kDecTcPassPrimes ? k - i0 : kDecTcPassPrimes;
-        if (tid == 0 && !failed) {
+        if (tid == 0) {
             // kind::i8: D s32 (bits 4-5 = 2), A and B u8, K-major; N >> 3 at bit 17, M >> 4 at bit 24
             const uint32_t ng = uint32_t((np + 1) & ~1);
             const uint32_t idesc = (2u << 4) | (ng << 17) | (uint32_t(kDecTcRows >> 4) << 24);
@@ -187,7 +178,7 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
                          : "memory");
         }
         // one warp polls, the others wait at the barrier
-        const bool ok = __syncthreads_and(warp != 0 || (!failed && mma_wait(smem_u32(&bar), uint32_t(g & 1))) ? 1 : 0) != 0;
+        ok = __syncthreads_and(warp != 0 || bar_wait(t, smem_u32(&bar), uint32_t(g & 1), kGiveUpMmas) ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int ib = i0 + 8 * half;
         const int ie = i0 + np < ib + 8 ? i0 + np : ib + 8;
@@ -208,27 +199,17 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
                     res_row(sB, i + 1)[res_slot(i + 1, m, C)] =
                         fold_planes(s + 8, uint32_t((uint64_t(1) << 62) - s_p[i + 1]));
             }
-        } else if (m < T) {
-            // the wait gave up: this warp's residues by the integer carry chains
-            const int n = (m >> logC) * N2 + j0 + (m & (C - 1));
-            const uint32_t* row = x + size_t(n) * size_t(L);
-            for (int i = ib; i < ie; ++i) {
-                uint32_t a0 = 0, a1 = 0, a2 = 0, b0 = 0, b1 = 0, b2 = 0;
-                for (int l = 0; l < L; ++l) {
-                    const uint64_t c = __ldg(t.pow32 + size_t(i) * kMaxL + l);
-                    mac_u32x64(__ldg(row + l), uint32_t(c), uint32_t(c >> 32), a0, a1, a2, b0, b1, b2);
-                }
-                res_row(sB, i)[res_slot(i, m, C)] =
-                    reduce_limb_sum(a0, a1, a2, b0, b1, b2, (uint64_t(1) << 62) - s_p[i]);
-            }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        failed = !ok;
         __syncthreads();  // this pass's reads are done before the next MMA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kDecTcCols) : "memory");
+    if (!ok) {
+        report_stuck(t);
+        return;
+    }
 
     // forward column stages of items (prime i, column j), then the residue rows
     if constexpr (LOG_N1 == 5) {

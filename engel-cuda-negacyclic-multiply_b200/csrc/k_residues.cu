@@ -215,6 +215,7 @@ __global__ void __launch_bounds__(128) k_residues_tc(TcArgs a) {
         }
     } else if (lane == 0) {
         atomicExch(a.status, 1u);
+        mbar_wait(smem_addr(bar), 0);  // late MMAs end before the tensor memory is given back
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

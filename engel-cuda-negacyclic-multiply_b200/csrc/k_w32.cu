@@ -21,10 +21,7 @@ namespace w32 {
 
 namespace {
 
-using crt_tc_detail::copy_polls;
 using crt_tc_detail::kmajor_desc;
-using crt_tc_detail::last_wait;
-using crt_tc_detail::mma_wait;
 using crt_tc_detail::smem_u32;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
@@ -226,7 +223,7 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
 
     for (int w = tid; w < 2 * wpairs; w += kThreads) {
         const PrimeConst32 pc = t.pc32[i0 + w];  // the MMAs' primes
-        s_pc[w] = make_uint2(pc.p, pc.bar >> 2);
+        s_pc[w] = make_uint2(pc.p, pc.c48);
     }
     if (early) pdl_trigger();
     pdl_wait();  // the operand and the residue rows belong to the stream's previous kernels
@@ -262,13 +259,8 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // (the thread of the MMAs has also waited for the weights; if that gave up, the residues go by the
-    // integer pipes, once the late copy has landed: they take its place)
-    bool failed = __syncthreads_or(tid == 0 && !mma_wait(smem_u32(&bars[1]), 0, copy_polls(t)) ? 1 : 0) != 0;
-    if (failed) {
-        if (tid == 0) last_wait(t, smem_u32(&bars[1]), 0);
-        __syncthreads();
-    }
+    // (the thread of the MMAs has also waited for the weights)
+    bool ok = __syncthreads_and(tid != 0 || bar_wait(t, smem_u32(&bars[1]), 0, kGiveUpCopies) ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
     const int slices = (kbytes + 31) / 32;
@@ -281,10 +273,10 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
     int slot[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) slot[e] = CC ? res_slot(e, m, CC) : 0;
-    for (int g = 0; g * kDecTc32PassPrimes < k; ++g) {
+    for (int g = 0; ok && g * kDecTc32PassPrimes < k; ++g) {
         const int ig = g * kDecTc32PassPrimes;
         const int np = k - ig < kDecTc32PassPrimes ? k - ig : kDecTc32PassPrimes;
-        if (tid == 0 && !failed) {
+        if (tid == 0) {
             const uint32_t ncols = uint32_t(((np + 3) & ~3) * 4);
             const uint32_t idesc = (2u << 4) | ((ncols >> 3) << 17) | (uint32_t(kDecTcRows >> 4) << 24);
             const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB + (ig >> 1) * 1024);
@@ -302,7 +294,7 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
                          : "memory");
         }
         // one warp polls, the others wait at the barrier (eight polling warps took an eighth of the issue slots)
-        const bool ok = __syncthreads_and(warp != 0 || (!failed && mma_wait(smem_u32(&bar), uint32_t(g & 1))) ? 1 : 0) != 0;
+        ok = __syncthreads_and(warp != 0 || bar_wait(t, smem_u32(&bar), uint32_t(g & 1), kGiveUpMmas) ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int ib = ig + 16 * half;
         const int ie = ig + np < ib + 16 ? ig + np : ib + 16;
@@ -329,25 +321,17 @@ __device__ __forceinline__ void dec_tc32_item(const ProductDesc& d, const Tables
                 for (int e = 0; e < 4; ++e)
                     rows[128 * e + (CC ? slot[e] : res_slot(i0 + i + e, m, C))] = fold_planes(s + 4 * e, p[e], c48[e]);
             }
-        } else if (m < T) {
-            // the wait gave up: this warp's residues on the integer pipes
-            const int n = (m >> logC) * N2 + j0 + (m & (C - 1));
-            const uint32_t* row = x + size_t(n) * size_t(L);
-            for (int i = ib; i < ie; ++i) {
-                const uint64_t p = s_pc[i].x;
-                uint64_t acc = 0;
-                for (int l = 0; l < L; ++l)
-                    acc = (acc + uint64_t(__ldg(row + l)) * __ldg(t.pow32_32 + size_t(i0 + i) * kMaxL + l)) % p;
-                res_row(sB, i)[res_slot(i0 + i, m, C)] = uint32_t(acc);
-            }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        failed = !ok;
         __syncthreads();  // this pass's reads are done before the next MMA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kDecTcCols) : "memory");
+    if (!ok) {
+        report_stuck(t);
+        return;
+    }
     dec32_columns<LOG_N1, CC, LN2>(R, t.fwd32, s_pc, sB, N, N2, logC, j0, i0, i1);
 }
 
@@ -609,52 +593,7 @@ __device__ __forceinline__ void crt32_finish(const QConst32* qc, const uint32_t*
     }
 }
 
-// The same coefficient (row u, column j) on the integer pipes, for a tile whose MMAs did not report
-// completion in time: the column sum from its definition, x_u N1 = sum_u' z_u' rho_u'^-2u with rho_u'
-// the forward twiddle of row block u' (node N1 + u'), then v_i = r_i y_i and the carry chains.
-template <int LW>
-__device__ __forceinline__ void crt32_coeff_plain(const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
-                                               const uint2* inv, int logN, int logN1, int k, int L, int u, int j,
-                                               uint32_t* out) {
-    constexpr int W = LW + kAccExtra;
-    const int N = 1 << logN, N2 = N >> logN1;
-    uint32_t acc[W], acc_hi[W];
-#pragma unroll
-    for (int w = 0; w < W; ++w) acc[w] = acc_hi[w] = 0;
-    uint64_t frac = 0;
-#pragma unroll 1
-    for (int i = 0; i < k; ++i) {
-        const uint64_t p = __ldg(&pc[i].p);
-        uint64_t x = 0;
-        for (int u2 = 0; u2 < (1 << logN1); ++u2) {
-            const uint64_t z = __ldcg(res + size_t(i) * N + size_t(u2) * N2 + j);
-            const uint64_t rho = __ldg(&inv[size_t(i) * kMaxN + (1 << logN1) + u2].x);
-            const uint64_t step = rho * rho % p;
-            uint64_t w = 1;
-            for (int e = 0; e < u; ++e) w = w * step % p;
-            x = (x + z * w) % p;
-        }
-        const uint32_t v = uint32_t(x * __ldg(qc->y + i) % p);
-        frac += (uint64_t(v) * __ldg(&pc[i].quo)) >> 29;
-        const uint32_t* M = qc->mq + i * kMqStride;
-        uint32_t m[LW];
-#pragma unroll
-        for (int l = 0; l < LW; ++l) m[l] = __ldg(M + l);
-        mac_lo<LW, 0, W>(acc, m, v);
-        mac_hi<LW, 1, W>(acc_hi, m, v);
-    }
-    mac_lo<LW, 0, W>(acc, qc->neg_m, uint32_t((frac + (1ull << 31)) >> 32));
-    mac_hi<LW, 1, W>(acc_hi, qc->neg_m, uint32_t((frac + (1ull << 31)) >> 32));
-    asm volatile("add.cc.u32 %0, %0, %1;" : "+r"(acc[0]) : "r"(acc_hi[0]));
-#pragma unroll
-    for (int w = 1; w < W - 1; ++w) asm volatile("addc.cc.u32 %0, %0, %1;" : "+r"(acc[w]) : "r"(acc_hi[w]));
-    asm volatile("addc.u32 %0, %0, %1;" : "+r"(acc[W - 1]) : "r"(acc_hi[W - 1]));
-    uint32_t r[LW + 1];
-    barrett<LW, W>(acc, qc->q, qc->mu, int(qc->qbits), r);
-    for (int l = 0; l < L; ++l) out[l] = r[l];
-}
-
-// Both by LW, not inlined: one copy serves the kernels of every column length, and at the call next to
+// By LW, not inlined: one copy serves the kernels of every column length, and at the call next to
 // nothing of theirs is live.
 __device__ __noinline__ void crt32_finish_any(int LW, const QConst32* qc, const uint32_t* s_consts, uint32_t lane_base,
                                               int L, uint32_t* o, bool store) {
@@ -663,18 +602,6 @@ __device__ __noinline__ void crt32_finish_any(int LW, const QConst32* qc, const 
     case n: crt32_finish<n>(qc, s_consts, lane_base, L, o, store); break;
         NC_LW_CASES(NC_CRT32_FINISH)
 #undef NC_CRT32_FINISH
-        default: break;
-    }
-}
-
-__device__ __noinline__ void crt32_plain_any(int LW, const uint32_t* res, const QConst32* qc, const PrimeConst32* pc,
-                                             const uint2* inv, int logN, int logN1, int k, int L, int u, int j,
-                                             uint32_t* out) {
-    switch (LW) {
-#define NC_CRT32_PLAIN(n) \
-    case n: crt32_coeff_plain<n>(res, qc, pc, inv, logN, logN1, k, L, u, j, out); break;
-        NC_LW_CASES(NC_CRT32_PLAIN)
-#undef NC_CRT32_PLAIN
         default: break;
     }
 }
@@ -705,9 +632,9 @@ __device__ __forceinline__ void crt32_store(uint32_t* c, int N2, int L, int j0, 
 
 // One tile with every thread of a 256-thread CTA, columns of 2^LOG_N1 points at stride 2^LN2 (N / N1
 // with LN2 0). The caller owns tensor-memory columns for the product's LW at `taddr` and
-// two initialised mbarriers `bars` (the MMAs', the table's).
+// two initialised mbarriers `bars` (the MMAs', the table's). False if one of them did not complete in time.
 template <int LOG_N1, int LN2>
-__device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
+__device__ __forceinline__ bool crt32_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, int logT,
                                                 bool early, uint8_t* smem, uint32_t taddr, uint64_t* bars) {
     uint64_t* bar = bars;
     using A = Crt32Layout<LOG_N1>;
@@ -747,13 +674,12 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
 
     const uint32_t bar_addr = smem_u32(bar);
     const int passes = (k + 31) >> 5;
-    bool ok = true;
-    int issued = 0;  // passes whose MMAs have been issued
 #pragma unroll 1
     for (int g = 0; g < passes; ++g) {
         // the A buffer is free once the pass before has been read
-        if (g > 0) ok = __syncthreads_and(warp != 0 || mma_wait(bar_addr, uint32_t((g - 1) & 1)) ? 1 : 0) != 0;
-        if (!ok) break;
+        if (g > 0 &&
+            !__syncthreads_and(warp != 0 || bar_wait(t, bar_addr, uint32_t((g - 1) & 1), kGiveUpMmas) ? 1 : 0))
+            return false;
         const int i0 = 32 * g, np = k - i0 < 32 ? k - i0 : 32;
         const uint32_t* res = ra + size_t(i0) * N + j0;
         constexpr int VJ = column_width(LOG_N1);
@@ -763,12 +689,7 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
             crt32_columns<LOG_N1, LN2, 1>(res, t.inv32 + size_t(i0) * kMaxN, logN, logC, np, s_p + i0, sA);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (g == 0)
-            ok = __syncthreads_and(tid != 0 || mma_wait(smem_u32(bars + 1), 0) ? 1 : 0) != 0;
-        else
-            __syncthreads();
-        if (!ok) break;
-        ++issued;
+        if (!__syncthreads_and(tid != 0 || g > 0 || bar_wait(t, smem_u32(bars + 1), 0, kGiveUpCopies) ? 1 : 0)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if (tid == 0) {
             const uint32_t idesc = (2u << 4) | (uint32_t(NC >> 3) << 17) | (uint32_t(kCrt32Rows >> 4) << 24);
@@ -786,26 +707,17 @@ __device__ __forceinline__ void crt32_coeffs_tc(const ProductDesc& d, const Tabl
                          : "memory");
         }
     }
-    ok = __syncthreads_and(ok && (warp != 0 || mma_wait(bar_addr, uint32_t((passes - 1) & 1))) ? 1 : 0) != 0;
+    if (!__syncthreads_and(warp != 0 || bar_wait(t, bar_addr, uint32_t((passes - 1) & 1), kGiveUpMmas) ? 1 : 0)) return false;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     // every MMA has read A: it takes the output tile
     uint32_t* s_out = reinterpret_cast<uint32_t*>(sA);
-    if (32 * warp < T) {
-        uint32_t* o = s_out + tid * L;
-        if (ok)
-            crt32_finish_any(LW, qc, s_negm, taddr + (uint32_t(32 * warp) << 16), L, o, tid < T);
-        else if (tid < T)
-            crt32_plain_any(LW, ra, qc, t.pc32, t.inv32, logN, LOG_N1, k, L, tid >> logC, j0 + (tid & (C - 1)), o);
-    }
+    if (32 * warp < T)
+        crt32_finish_any(LW, qc, s_negm, taddr + (uint32_t(32 * warp) << 16), L, s_out + tid * L, tid < T);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     crt32_store(c_out, N2, L, j0, C, 1 << LOG_N1, s_out);
-    if (!ok) {
-        // late copies and MMAs end (bounded) before the memory they write is given back
-        mma_wait(smem_u32(bars + 1), 0);
-        if (issued > 0) mma_wait(bar_addr, uint32_t((issued - 1) & 1));
-    }
+    return true;
 }
 
 // The tile within a kernel: tensor memory (`cols` columns) and the mbarrier around it.
@@ -830,10 +742,10 @@ __device__ __forceinline__ void crt32_cta(const ProductDesc& d, const Tables& t,
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t taddr = taddr_slot;
-    if (LOG_N1 <= 4 && d.logN == 12 + LOG_N1)
-        crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, early, smem, taddr, bars);
-    else
-        crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, early, smem, taddr, bars);
+    const bool ok = LOG_N1 <= 4 && d.logN == 12 + LOG_N1
+                        ? crt32_coeffs_tc<LOG_N1, 12>(d, t, tile, logT, early, smem, taddr, bars)
+                        : crt32_coeffs_tc<LOG_N1, 0>(d, t, tile, logT, early, smem, taddr, bars);
+    if (!ok) report_stuck(t);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (threadIdx.x < 32)

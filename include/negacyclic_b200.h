@@ -25,7 +25,8 @@ enum {
     NC_EINVAL = -1,   /* bad argument: size, alignment, modulus, null pointer */
     NC_ECUDA = -2,    /* a CUDA call failed */
     NC_ENOMEM = -3,   /* device or pinned allocation failed, or an HBM budget is exceeded */
-    NC_ETIMEOUT = -4, /* a persistent-kernel dependency wait gave up (bounded spin) */
+    NC_ETIMEOUT = -4, /* a kernel's bounded wait ran out: a batch's dependency, or a copy or MMAs of its
+                         own (then every later call on the device returns it too) */
     NC_EBUSY = -5,    /* the object is in use (server full, request not finished) */
     NC_ESELFCHECK = -6 /* an init-time self-check failed (host arithmetic, tables, plan constants,
                           or the device's known-answer product) */
