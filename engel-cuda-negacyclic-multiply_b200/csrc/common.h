@@ -180,8 +180,9 @@ struct Tables {
     // builds the word's address carries kGiveUp bits.
     uint32_t* stuck;
 };
-// NC_TEST_GIVE_UP builds: waits for copies, and waits for MMAs, that count as run out once they are over.
-enum : uint32_t { kGiveUpCopies = 1, kGiveUpMmas = 2, kGiveUpBits = 3 };
+// NC_TEST_GIVE_UP builds: waits that count as run out once they are over (for tables, for MMAs, for a row
+// block's twiddles and residues).
+enum : uint32_t { kGiveUpCopies = 1, kGiveUpMmas = 2, kGiveUpRows = 4, kGiveUpBits = 7 };
 
 // Dynamic shared memory of each stage.
 NC_HD constexpr size_t smax(size_t a, size_t b) { return a > b ? a : b; }

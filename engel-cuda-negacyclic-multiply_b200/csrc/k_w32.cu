@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3
     if (early) pdl_trigger();
     const uint32_t b = smem_u32(&bar);
     w32::row_barrier_init<LOG_N2, LOG_E, THREADS>(b);
-    w32::row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem, b, 0, true, true);
+    if (!w32::row_blocks<LOG_N2, LOG_E, THREADS>(d, t, int(blockIdx.x), smem, b, 0, true)) report_stuck(t);
 }
 
 #define NC_ROW32_VARIANTS(X)                                                                                   \
@@ -807,10 +807,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_batch_dec_tc32(BatchCrtArgs a) 
 
 // Row items (x = product, y = row-CTA index) with row blocks of 2^LOG_N2, radix 8, 256 threads:
 // persistent CTAs take items in queue order; each item's twiddles and residue blocks arrive on the
-// CTA's mbarrier, one phase per item. If a bulk wait gives up (the item then loads its data with
-// plain loads), the CTA's later items use plain loads too. Bound as k_row32 is, without its last wave
-// (64 x 16384, 868 bits: 481 -> 437 us with padded places, block barriers and additions off the
-// multiply pipe).
+// CTA's mbarrier, one phase per item. Bound as k_row32 is, without its last wave (64 x 16384, 868 bits:
+// 481 -> 437 us with padded places, block barriers and additions off the multiply pipe).
 template <int LOG_N2>
 __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -825,7 +823,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) 
     const uint32_t b = smem_u32(&bar);
     row_barrier_init<LOG_N2, kBatchRowLogE, kThreads>(b);
     uint32_t parity = 0;
-    bool bulk = true;
+    bool ok = true;
     auto load_product = [&](uint32_t x) {
         if (threadIdx.x < kWords)
             reinterpret_cast<uint32_t*>(&s_bp)[threadIdx.x] =
@@ -833,9 +831,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) 
         __syncthreads();
     };
     auto single = [&](int y) {
-        const bool ok = row_blocks<LOG_N2, kBatchRowLogE, kThreads>(s_bp.d, a.tables, y, smem, b, parity, bulk);
-        if (bulk) parity ^= 1u;
-        bulk = bulk && ok;  // the item's result stands either way; later items avoid the barrier
+        ok = row_blocks<LOG_N2, kBatchRowLogE, kThreads>(s_bp.d, a.tables, y, smem, b, parity);
+        parity ^= 1u;
     };
     for (;;) {
         if (threadIdx.x == 0) s_item = int(atomicAdd(a.head, kPairs ? 2u : 1u));
@@ -851,12 +848,11 @@ __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) 
             const int mask = (1 << logN1) - 1;
             const int mirror = (int(w.y) & ~mask) | (mask - (int(w.y) & mask));
             if (has2 && w2.x == w.x && s_bp.d.mode == kModeProduct && logN1 >= 1 && int(w2.y) == mirror) {
-                // two phases when the copies ran, so the parity is unchanged
-                bulk = row_pair<LOG_N2, kBatchRowLogE, kThreads>(s_bp.d, a.tables, int(w.y), int(w2.y), smem, b, parity,
-                                                                 bulk, a.error, w.x);
+                // two phases, so the parity is unchanged
+                ok = row_pair<LOG_N2, kBatchRowLogE, kThreads>(s_bp.d, a.tables, int(w.y), int(w2.y), smem, b, parity);
             } else {
                 single(int(w.y));
-                if (has2) {
+                if (ok && has2) {
                     __syncthreads();  // s_bp is rewritten
                     load_product(w2.x);
                     single(int(w2.y));
@@ -864,6 +860,10 @@ __global__ void __launch_bounds__(kThreads, 4) k_persistent_rows32(BatchArgs a) 
             }
         } else {
             single(int(w.y));
+        }
+        if (!ok) {
+            report_stuck(a.tables);
+            break;
         }
         __syncthreads();  // s_item and s_bp are rewritten by the next round
     }

@@ -332,26 +332,10 @@ NC_HD constexpr size_t row_smem_bytes(int threads, int logE) {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// Bounded wait for phase `parity` of the mbarrier at shared address `bar`: false if it did not
-// complete within 2^22 polls. cta_wait is the whole CTA's: one warp polls and the rest wait at the
-// barrier (every warp polling took a sixth of the row kernel's instructions).
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity) {
-    for (uint32_t it = 0; it < (1u << 22); ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
-}
-
-__device__ __forceinline__ bool cta_wait(uint32_t bar, uint32_t parity) {
-    return __syncthreads_and(threadIdx.x >= 32 || bar_wait(bar, parity) ? 1 : 0) != 0;
+// The CTA's bounded wait for the copies of phase `parity` of its mbarrier: one warp polls and the rest wait
+// at the barrier (every warp polling took a sixth of the row kernel's instructions).
+__device__ __forceinline__ bool cta_wait(const Tables& t, uint32_t bar, uint32_t parity) {
+    return __syncthreads_and(threadIdx.x >= 32 || bar_wait(t, bar, parity, kGiveUpRows) ? 1 : 0) != 0;
 }
 
 // The twiddles of the row block under node `base` of the merged tree: local stage l uses the 2^l
@@ -370,26 +354,15 @@ __device__ __forceinline__ void stage_twiddles(const uint2* tw, int base, uint2*
                      : "memory");
 }
 
-// The same entries by plain loads, every thread of the CTA taking its share (the fallback if the
-// bulk copies do not complete in time).
-template <int LOG_N2>
-__device__ __forceinline__ void copy_twiddles(const uint2* tw, int base, uint2* s, int part, int parts) {
-    for (int e = 1 + part; e < (1 << LOG_N2); e += parts) {
-        const int l = 31 - __clz(e);
-        s[e] = __ldg(tw + (size_t(base) << l) + (e - (1 << l)));
-    }
-}
-
 // One CTA of THREADS threads handles THREADS / T row blocks, as row_blocks of stages.cuh: block
 // rb = item * ROWS + (tid / T) is prime rb >> logN1, row u = rb & (N1 - 1). Modes: product
 // (forward a and b, pointwise, inverse), cached-a (a's transform read from a_hat), forward (a's
 // transform written to hat_out). Residues are k x N u32. The twiddles and the residue blocks of
 // each row block are staged in shared memory at the start by bulk copies that complete on the
 // CTA's mbarrier `bar` (row_barrier_init), phase `parity` (a persistent CTA's items alternate
-// phases): the passes then wait on no global load. use_bulk false (a persistent CTA after a bulk
-// wait gave up) loads them with plain loads instead. Returns false if this item's bulk wait gave
-// up (its data then came by plain loads, so the item's result stands). With `trigger`, the next kernel
-// may be scheduled once the residues are there (a kernel of one item a CTA).
+// phases): the passes then wait on no global load. Returns false, with nothing written, if the copies did
+// not land in time (the CTA then ends). With `trigger`, the next kernel may be scheduled once the residues
+// are there (a kernel of one item a CTA).
 template <int LOG_N2, int LOG_E, int THREADS>
 __device__ __forceinline__ void row_barrier_init(uint32_t bar) {
     using S = RowShape<LOG_N2, LOG_E>;
@@ -406,7 +379,7 @@ __device__ __forceinline__ void row_barrier_init(uint32_t bar) {
 
 template <int LOG_N2, int LOG_E, int THREADS>
 __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t, int item, uint8_t* smem,
-                                           uint32_t bar, uint32_t parity, bool use_bulk, bool trigger = false) {
+                                           uint32_t bar, uint32_t parity, bool trigger = false) {
     using S = RowShape<LOG_N2, LOG_E>;
     static_assert(S::T <= THREADS, "row block needs more threads than the CTA has");
     constexpr int ROWS = THREADS / S::T;
@@ -440,29 +413,13 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
     uint32_t v[S::E];
 
     __syncthreads();  // shared memory of a previous item is free
-    if (use_bulk && lt == 0) {
+    if (lt == 0) {
         // the twiddle tables do not depend on the previous kernel: their copies start before its end
         const uint32_t bytes = (inverse ? 2u : 1u) * 8u * ((1u << LOG_N2) - 2u);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
         stage_twiddles<LOG_N2>(twf, base, s_twf, bar);
         if (inverse) stage_twiddles<LOG_N2>(twf, base_mirror, s_twi, bar);
     }
-    // the CTA waits for the copies (bounded); if that gave up, each row's threads copy its
-    // twiddles themselves and, before the item ends, wait once more for the copies in flight
-    bool staged = use_bulk;
-    auto twiddles_ready = [&] {
-        if (use_bulk) staged = cta_wait(bar, parity);
-        if (!staged) {
-            copy_twiddles<LOG_N2>(twf, base, s_twf, lt, S::T);
-            if (inverse) copy_twiddles<LOG_N2>(twf, base_mirror, s_twi, lt, S::T);
-            __syncthreads();
-        }
-    };
-    auto finish = [&] {
-        if (use_bulk && !staged) bar_wait(bar, parity);
-        return staged || !use_bulk;
-    };
-
     pdl_wait();  // the residues come from the stream's previous kernel
     if (trigger) pdl_trigger();
     // the residue blocks as bulk copies too (16-byte aligned for blocks of 4 and more): product
@@ -474,7 +431,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
     uint32_t* a_dst = d.mode == kModeCachedA ? buf : buf_a;
     uint32_t* b_dst = d.mode == kModeCachedA ? buf_a : b_in;
     const bool b_bulk = d.mode == kModeCachedA || (PF_B && d.mode == kModeProduct);
-    if (BULK && use_bulk && lt == 0) {
+    if (BULK && lt == 0) {
         asm volatile("fence.proxy.async.global;" ::: "memory");  // the previous kernel's writes -> bulk reads
         const uint32_t bytes = (b_bulk ? 2u : 1u) * 4u * uint32_t(S::N2);
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -497,15 +454,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
             if (b_bulk) b_dst[x] = __ldcg(rb_res + off + x);
         }
     }
-    twiddles_ready();
-    if (BULK && !staged) {
-        // no bulk copies, or they gave up: each row's threads load its blocks themselves
-        for (int x = lt; x < S::N2; x += S::T) {
-            a_dst[x] = __ldcg(a_src + x);
-            if (b_bulk) b_dst[x] = __ldcg(rb_res + off + x);
-        }
-        __syncthreads();
-    }
+    if (!cta_wait(t, bar, parity)) return false;
     if (d.mode == kModeCachedA) {
         // b's residues to registers, then a_hat from its raw block into buf_a in the last pass's
         // swizzled layout (b's raw block, also in buf_a, is read first)
@@ -534,7 +483,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
 #pragma unroll
                 for (int e = 0; e < S::E; ++e) __stcg(out + off + row_index<S, 0>(lt, e), v[e]);
             }
-            return finish();
+            return true;
         }
         row_store<S, LAST>(v, buf_a, lt);
         if constexpr (PF_B) {
@@ -559,7 +508,7 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
 #pragma unroll
         for (int e = 0; e < S::E; ++e) __stcg(out + off + row_index<S, 0>(lt, e), v[e]);
     }
-    return finish();
+    return true;
 }
 
 // Row pairs of a batch's persistent row launch (plain products, one row block a row of the CTA):
@@ -570,14 +519,10 @@ __device__ __forceinline__ bool row_blocks(const ProductDesc& d, const Tables& t
 // Mbarrier phases (two arrivals each, row_barrier_init): `parity` for the twiddles and u's block
 // of a, parity ^ 1 for the block of a of u'; b's blocks come by plain loads in the forward pass,
 // as in row_blocks without row_prefetch_b (256-thread CTAs). rb0 and rb1 are the two row blocks
-// (prime * N1 + u). Returns false if a bulk wait gave up (the blocks then came by
-// plain loads and the results stand); the caller then stops using the barrier. With use_bulk
-// false every block comes by plain loads. If the first member's copies have not landed after two
-// bounded waits, its buffers cannot safely take the second member's blocks: error[0] is set
-// (error[1] = what), which the host reports as a failed batch.
+// (prime * N1 + u). Returns false if copies did not land in time (the CTA then ends).
 template <int LOG_N2, int LOG_E, int THREADS>
 __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, int rb0, int rb1, uint8_t* smem,
-                                         uint32_t bar, uint32_t parity, bool use_bulk, uint32_t* error, uint32_t what) {
+                                         uint32_t bar, uint32_t parity) {
     using S = RowShape<LOG_N2, LOG_E>;
     static_assert(S::T == THREADS && LOG_N2 >= 2, "row pairs take one row block a CTA, staged by bulk copies");
     static_assert(!row_prefetch_b(THREADS), "row pairs load b's blocks in the forward pass");
@@ -605,13 +550,9 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
                      "l"(ra + off), "r"(4u * S::N2), "r"(bar)
                      : "memory");
     };
-    // the same block by plain loads, every thread
-    auto load_blocks = [&](size_t off) {
-        for (int x = lt; x < S::N2; x += S::T) buf_a[x] = __ldcg(ra + off + x);
-    };
 
     __syncthreads();  // shared memory of a previous item is free
-    if (use_bulk && lt == 0) {
+    if (lt == 0) {
         // the twiddles do not depend on the previous kernel: their copies start before its end
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16u * ((1u << LOG_N2) - 2u))
                      : "memory");
@@ -619,40 +560,16 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
         stage_twiddles<LOG_N2>(twf, (1 << logN1) + u1, s_tw1, bar);
     }
     pdl_wait();  // the residues come from the stream's previous kernel
-    if (use_bulk && lt == 0) {
+    if (lt == 0) {
         asm volatile("fence.proxy.async.global;" ::: "memory");  // the previous kernel's writes -> bulk reads
         copy_blocks(off0);
     }
-    // phase whose copies may still be in flight (-1: none) once a wait gave up
-    int pending = -1;
-    bool staged = use_bulk && cta_wait(bar, parity);
-    if (!staged) {
-        if (use_bulk) pending = 0;
-        copy_twiddles<LOG_N2>(twf, (1 << logN1) + u0, s_tw0, lt, S::T);
-        copy_twiddles<LOG_N2>(twf, (1 << logN1) + u1, s_tw1, lt, S::T);
-        load_blocks(off0);
-        __syncthreads();
-    }
+    if (!cta_wait(t, bar, parity)) return false;
     const uint32_t p2 = 2 * p;
 #pragma unroll 1
     for (int j = 0; j < 2; ++j) {
         const size_t off = j ? off1 : off0;
-        if (j == 1) {
-            if (staged) {
-                staged = cta_wait(bar, parity ^ 1u);
-                if (!staged) pending = 1;
-            } else if (pending == 0) {
-                // once the late copies of the first member are done, its buffers are free
-                if (cta_wait(bar, parity))
-                    pending = -1;
-                else if (error && lt == 0 && atomicCAS(error, 0u, 1u) == 0u)
-                    error[1] = what;
-            }
-            if (!staged) {
-                load_blocks(off1);
-                __syncthreads();
-            }
-        }
+        if (j == 1 && !cta_wait(t, bar, parity ^ 1u)) return false;
         uint32_t v[S::E];
 #pragma unroll
         for (int e = 0; e < S::E; ++e) v[e] = buf_a[row_index<S, 0>(lt, e)];
@@ -670,7 +587,7 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
         }
         if (j == 0) {
             __syncthreads();  // every thread has read buf_a
-            if (staged && lt == 0) {
+            if (lt == 0) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // those reads -> the bulk writes
                 copy_blocks(off1);
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -680,8 +597,7 @@ __device__ __forceinline__ bool row_pair(const ProductDesc& d, const Tables& t, 
 #pragma unroll
         for (int e = 0; e < S::E; ++e) __stcg(out + off + row_index<S, 0>(lt, e), v[e]);
     }
-    if (pending >= 0) bar_wait(bar, pending ? parity ^ 1u : parity);  // copies in flight end before the smem is reused
-    return use_bulk && pending < 0;
+    return true;
 }
 
 }  // namespace w32
