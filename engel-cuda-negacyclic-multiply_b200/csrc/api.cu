@@ -166,7 +166,7 @@ int nc_plan_set_residue_engine(nc_plan* plan, int engine) {
         if (engine != NC_RESIDUES_IMAD && engine != NC_RESIDUES_TC_I8) throw nc::Error(nc::kEInval, "unknown residue engine");
         if (engine == NC_RESIDUES_TC_I8 && !plan->p->tables->tensor_cores)
             throw nc::Error(nc::kEInval, "the tensor-core residue stage needs a compute capability 10.0 device");
-        plan->p->res_tc = engine == NC_RESIDUES_TC_I8;
+        nc::plan_set_residue_engine(plan->p, engine == NC_RESIDUES_TC_I8);
     });
 }
 

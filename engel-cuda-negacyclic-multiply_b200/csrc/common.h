@@ -241,9 +241,13 @@ constexpr int kRowLogCap = 13;
 // The 62-bit engine's row configuration before any tuning: radix-8 passes on blocks of N / 8, 2^6 to
 // 2^11 residues (us a product, blocks of min(N, 2^12) with radix-16 passes against these: 434 bits,
 // N = 2048 42.3 and 23.2, N = 65536 77.3 and 74.0; 1000 bits, N = 1024 65.0 and 46.0, N = 65536 219 and
-// 178; three operands of 868 bits, N = 16384 125 and 99); radix 16 below, where radix 8 has no kernel.
-inline RowConfig default_row_config(int logN) {
+// 178); radix 16 below, where radix 8 has no kernel. With residues on the integer pipes, blocks of 2^12 at
+// N = 2^16 up to 18 primes, where 16-point columns gain more than the rows lose (blocks of 2^12 and of
+// 2^11: 434 bits, 15 primes 82.0 and 94.2; 530 bits, 18 primes 96.3 and 105.4; 560 bits, 19 primes 119.3
+// and 116.3).
+inline RowConfig default_row_config(int logN, int k, bool res_tc) {
     if (logN < 6) return RowConfig{logN, 4, 256};
+    if (logN == kMaxLogN && !res_tc && k <= 18) return RowConfig{12, 3, 512};
     const int block = logN - 3;
     return RowConfig{block < 6 ? 6 : block > 11 ? 11 : block, 3, 256};
 }

@@ -351,7 +351,7 @@ Plan* plan_create(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int fac
         throw Error(kESelfCheck, "init self-check of the plan's constants: " + qerr);
     }
     p->k = int(p->hq.k);
-    if (!tuned_row_config(logN, int(L), &p->cfg)) p->cfg = default_row_config(logN);
+    p->cfg_default = !tuned_row_config(logN, int(L), &p->cfg);
     // the 30-bit engine: pairs whose bound fits its 64 primes
     bool w32_consts = false;
     if (factors == 2 && build_qconst32(q, int(L), logN, &p->hq32).empty()) {
@@ -370,6 +370,7 @@ Plan* plan_create(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, int fac
         p->device = current_device();
         p->tables = acquire_tables(p->device);
         if (!p->tables->tensor_cores) p->res_tc = p->crt_tc = false;  // integer-pipe engines only
+        if (p->cfg_default) p->cfg = default_row_config(logN, p->k, p->res_tc);
         check(cudaMalloc(&p->d_qc, sizeof(QConst)), "plan constants");
         check(cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking), "stream");
         // ordered on the plan's stream and complete before any other stream can use the plan
@@ -917,6 +918,12 @@ void plan_set_row_config(Plan* p, const RowConfig& c) {
     if (!row_config_valid(p->logN, c) || !row_variant_exists(c))
         throw Error(kEInval, "no compiled row kernel for this configuration and N");
     p->cfg = c;
+    p->cfg_default = false;
+}
+
+void plan_set_residue_engine(Plan* p, bool tensor_cores) {
+    p->res_tc = tensor_cores;
+    if (p->cfg_default) p->cfg = default_row_config(p->logN, p->k, p->res_tc);
 }
 
 void plan_set_word_bits(Plan* p, int bits) {
@@ -977,6 +984,7 @@ float plan_autotune(Plan* p, int reps) {
         }
     }
     p->cfg = best;
+    p->cfg_default = false;
     // the 30-bit engine's, where it can run; the faster engine is kept
     const bool try32 = p->w32_ok && p->res_tc && p->crt_tc && !word64_forced();
     RowConfig best32 = p->cfg32;

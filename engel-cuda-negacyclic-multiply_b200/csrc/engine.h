@@ -121,6 +121,7 @@ struct Plan {
     HostPool* pool = nullptr;
     float last_kernel_ms = 0.f;
     RowConfig cfg{};                 // row-stage tiling of the plain path (autotuned per N)
+    bool cfg_default = true;         // it is default_row_config's, and follows the residue engine
     uint4* d_crt_b = nullptr;        // byte table of the tensor-core CRT (k <= 32), built at creation
     bool crt_tc = true;              // plain path: CRT accumulation on the tensor cores when available
     bool res_tc = true;              // plain path: residue stage on the tensor cores
@@ -186,6 +187,7 @@ int current_device();
 
 // Row configuration for the plain path of a plan: validated and applied.
 void plan_set_row_config(Plan* p, const RowConfig& c);
+void plan_set_residue_engine(Plan* p, bool tensor_cores);
 
 // Times every compiled row configuration valid for the plan's N on its own buffers (`reps`
 // products each, device-resident), applies the fastest and remembers it for later plans of
