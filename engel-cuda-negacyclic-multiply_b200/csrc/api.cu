@@ -80,7 +80,8 @@ int nc_self_check(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q) {
         // the 30-bit engine's constants, where its 64 primes cover the bound
         nc::QConst32 c32{};
         if (nc::build_qconst32(q, int(L), logN, &c32).empty()) {
-            const std::string e32 = nc::check_qconst32(c32);
+            std::string e32 = nc::check_qconst32(c32);
+            if (e32.empty()) e32 = nc::check_crt32_table(c32, nc::crt32_table(c32));
             if (!e32.empty()) throw nc::Error(nc::kESelfCheck, "init self-check of the plan's 30-bit constants: " + e32);
         }
     });

@@ -601,7 +601,8 @@ std::string check_prime_set32() {
         const std::string at = "30-bit prime " + std::to_string(i) + ": ";
         if (!is_prime64(c.p)) return at + "composite";
         if (((c.p - 1) & ((1u << kRootLog) - 1)) != 0) return at + "not 1 mod 2^17";
-        if (c.p >= (1u << 30) || c.p <= (1u << 29)) return at + "not in (2^29, 2^30)";
+        // (fold_planes needs p > 0.81 2^30 for residues below 4p)
+        if (c.p >= (1u << 30) || c.p <= (7u << 27)) return at + "not in (7/8 2^30, 2^30)";
         if (uint32_t(c.p * (0u - c.pinv)) != 1u) return at + "pinv is not -p^-1 mod 2^32";
         if (uint64_t(c.c48) != (1ull << 48) / c.p) return at + "reciprocal constant";
         if (i > 0 && c.p >= ps[size_t(i) - 1].p) return "30-bit prime set not descending";
@@ -744,11 +745,54 @@ std::string check_qconst32(const QConst32& c) {
     const Big e1 = pow2(int(c.qbits) + 31);
     if (bits_of(qb) > 1 && (cmp_big(mul_big(m1, qb), e1) > 0 || cmp_big(add_big(mul_big(m1, qb), qb), e1) <= 0))
         return "one-word quotient constant";
+    if (bits_of(qb) == 1 && c.mu1 != 0xffffffffu) return "one-word quotient constant";
     uint64_t carry = 0;
     for (int l = 0; l <= int(c.LW); ++l) {
         carry += uint64_t(c.neg_q[l]) + c.q[l];
         if (uint32_t(carry) != 0) return "two's complement of q";
         carry >>= 32;
+    }
+    // the quotient's window: five bytes that hold q's leading bits, 31 of them after the shift
+    const int c0 = int(c.top_byte);
+    if (c0 != std::max(0, (int(c.qbits) - 1) / 8 - 4)) return "first byte of the quotient's window";
+    if (8 * c0 + c.top_shift + 14 != int(c.qbits)) return "shift of the quotient's window";
+    Big window = neg;  // floor(((-M) mod q) / 2^(8 c0))
+    Big byte{256};
+    for (int b = 0; b < c0; ++b) {
+        Big up;
+        divmod(window, byte, &up);
+        window = up;
+    }
+    window.resize(std::max<size_t>(window.size(), 2), 0);
+    if (window.size() != 2 || ((uint64_t(window[1]) << 32) | window[0]) != c.top_neg_m)
+        return "(-M) mod q in the quotient's window";
+    return std::string();
+}
+
+std::string check_crt32_table(const QConst32& c, const std::vector<uint8_t>& b) {
+    const int LW = int(c.LW), k = int(c.k), NC = crt32_cols(LW);
+    const auto& ps = prime_set32();
+    if (b.size() != crt32_table_bytes(LW)) return "size of the CRT table";
+    Big qb(c.q, c.q + c.L), neg(c.neg_m, c.neg_m + kMqStride);
+    trim(qb);
+    trim(neg);
+    for (int K = 0; K < 256; ++K) {
+        const std::string at = "CRT table row " + std::to_string(K) + ": ";
+        std::vector<uint32_t> row(size_t(NC) / 4, 0);
+        for (int col = 0; col < NC; ++col)
+            row[size_t(col / 4)] |= uint32_t(b[size_t(col / 8) * 2048 + size_t(K / 16) * 128 + size_t(col % 8) * 16 + size_t(K % 16)])
+                                    << (8 * (col % 4));
+        for (int w = K < 4 * k ? LW + 1 : 0; w < NC / 4; ++w)
+            if (row[size_t(w)] != 0) return at + "not zero beyond its weight";
+        if (K >= 4 * k) continue;
+        // weight E < q with E p_i + ((-M) mod q) w = 0 (mod q), w = 2^(8a) y_i mod p_i, and floor(2^32 w / p_i)
+        const uint64_t p = ps[size_t(K / 4)].p;
+        const uint64_t w = mulmod64(c.y[K / 4], powmod64(2, uint64_t(8 * (K % 4)), p), p);
+        Big e(row.begin(), row.begin() + LW);
+        trim(e);
+        if (cmp_big(e, qb) >= 0) return at + "weight not below q";
+        if (!divmod(add_big(mul_u64(e, p), mul_u64(neg, w)), qb, nullptr).empty()) return at + "weight";
+        if (row[size_t(LW)] != uint32_t((w << 32) / p)) return at + "share of the quotient";
     }
     return std::string();
 }

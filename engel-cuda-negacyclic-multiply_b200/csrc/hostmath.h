@@ -72,7 +72,8 @@ std::vector<uint8_t> crt32_table(const QConst32& c);
 
 std::string check_prime_set32();                                 // primes, 1 mod 2^17, constants
 std::string check_tables32(const HostTables32& t, int samples);  // psi, sampled twiddles
-std::string check_qconst32(const QConst32& c);                   // CRT identities and mu
+std::string check_qconst32(const QConst32& c);                   // CRT identities, the one-word quotient's constants
+std::string check_crt32_table(const QConst32& c, const std::vector<uint8_t>& b);  // every weight and quotient byte
 
 // c = a * b mod (X^N + 1, q) by the schoolbook sum on big integers (small N only: the device
 // self-test's expected answer).

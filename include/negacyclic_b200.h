@@ -53,8 +53,10 @@ int nc_plan_create(uint32_t N, uint32_t W, uint32_t L, const uint32_t* q, nc_pla
    the plan's CRT constants: y_i (M/p_i) N = 1 mod p_i from an independent product of the other
    primes, (M/p_i mod q) p_i + ((-M) mod q) = 0 mod q for every i, the Barrett constant's defining
    inequality, and the Shoup companions; the same for the 30-bit word engine's constants where its
-   primes cover the bound (y_i (M/p_i) N = 2^32 mod p_i). They hold for every valid q. Returns NC_OK, NC_EINVAL for
-   an invalid point, or NC_ESELFCHECK. nc_plan_create runs the same checks and, once per device,
+   primes cover the bound (y_i (M/p_i) N = 2^32 mod p_i, and the constants of the one-word quotient by
+   q), and every weight and quotient byte of its CRT table. They hold for every valid q. Returns NC_OK,
+   NC_EINVAL for an invalid point, or NC_ESELFCHECK. nc_plan_create runs the same checks but the
+   table's and, once per device,
    an N = 8 known-answer product on the device. Mirrors the self-checks of the reference's
    fherma_init (solve.cu:1151-1165, 1285-1314, 1370-1415), without its L = 28 Barrett check,
    which rejects nearly every 868-bit q. */
