@@ -644,10 +644,13 @@ std::vector<std::pair<size_t, size_t>> download_chunks(size_t bytes) {
 
 // Operand b of a pair goes up in this many column groups, each a strided copy of its columns of
 // every row segment, and each group's residue tiles start as soon as it has landed: the residue
-// stage of b then ends about one group's tiles after the last byte, not a whole stage after.
+// stage of b then ends about one group's tiles after the last byte, not a whole stage after. From
+// 7 MiB an operand; below, the copies, events and launches of four groups cost more than that (us a
+// host product, four groups and one: N = 2^13, 1000 bits 205 and 163; 2^14, 434 bits 138 and 126; 2^15,
+// 868 bits 349 and 343; 2^16, 434 bits 346 and 336, 868 bits 561 and 561, 1000 bits 701 and 713).
 int upload_groups(const Plan* p, const ProductDesc& d) {
     constexpr int kGroups = 4;
-    if (p->N < (1 << 13)) return 1;
+    if (p->limbs() * sizeof(uint32_t) < size_t(7) << 20) return 1;
     return residue_tiles(d, p->plain_cfg()) % kGroups == 0 ? kGroups : 1;
 }
 
