@@ -43,11 +43,13 @@ __device__ __forceinline__ void report_stuck(const Tables& t) {
     *reinterpret_cast<volatile uint32_t*>(reinterpret_cast<uintptr_t>(t.stuck) & ~uintptr_t(kGiveUpBits)) = 1;
 }
 
-// Programmatic dependent launch. A product kernel launched with it may be scheduled while the
-// kernel before it on the stream still runs (once every CTA of that kernel has called
-// pdl_trigger(): after its own pdl_wait() in the product kernels, so that the CTAs of two products
-// are never queued together, and once the CTA holds its tensor memory), so its prologue (tensor-memory allocation, constant tables) overlaps that
-// kernel's last wave.
+// Programmatic dependent launch. A product kernel launched with it may be scheduled while the kernel
+// before it on the stream still runs (once every CTA of that kernel has called pdl_trigger() or ended), so
+// its prologue (tensor-memory allocation, constant tables) overlaps that kernel's last wave. A kernel that
+// holds tensor memory triggers only once its CTA has it. Most trigger after their own pdl_wait(), so that
+// the CTAs of two products are never queued together; short 30-bit kernels (early_triggers, k_w32.cu), the
+// integer-pipe residues (k_dec) and the row and CRT launches of batches (k_batch.cu, k_persistent_rows32)
+// trigger before it: a batch's next launch has the CTAs of its own products only.
 // pdl_wait() returns once the kernel before has completed and its writes are visible; every read
 // or write of data that kernel produces or consumes comes after it. In a kernel launched without
 // the attribute, both return at once.

@@ -11,16 +11,15 @@
 
 namespace nc {
 
-
 // A list of products (each referring to a plan for its q, N and constants) that run together.
 // Products may differ in N and in q. Residue scratch comes from the batch's own arena. A run is,
 // for products below N = 2^15: the tensor-core residue launches, one persistent launch for the
 // row stage (and any residue items on the integer pipes), then the CRT launches of the engines in
 // use. Products of N >= 2^15 fill the GPU on their own: they run the plain path's launches with
 // their plan's row configuration, alternating between two streams so that one product's last
-// wave overlaps the next one's kernels. Plain products (a, b -> c) of plans on the 30-bit word
-// engine run on it (residue scratch from the batch's arena): below 2^15 in their own residue,
-// persistent-row and CRT launches (one per column length) after the 62-bit ones, from 2^15 as the plain path's launches.
+// wave overlaps the next one's kernels. Products of plans on the 30-bit word engine run on it
+// (residue scratch from the batch's arena): below 2^15 in their own residue, persistent-row and CRT
+// launches (one per column length) after the 62-bit ones, from 2^15 as the plain path's launches.
 // The counter reset and the launches are captured once into a CUDA graph and replayed while the
 // batch keeps the same shape.
 class Batch {

@@ -135,9 +135,10 @@ struct QConst32 {
 // The 30-bit engine's tensor-core CRT: 128-coefficient tiles (one MMA's M) from N = 2^15, 64 below and
 // 32 up to 2^11 while a row segment still holds eight columns: a CTA walks its primes x columns one
 // after another, so at small N more and shorter CTAs win (868 bits, us a product: N = 16384 25.0 with 64,
-// 26.7 with 128; N = 32768 38.4 and 38.3; N = 1024 13.3 with 32, 14.0 with 64; 434 bits, N = 16384 21.6
-// with 64, 20.5 with 128). The table B has the 4 LW bytes of a coefficient sum and
-// 4 bytes of the quotient sum as columns; its accumulator takes a power of two of tensor-memory columns.
+// 26.7 with 128; N = 32768 38.4 and 38.3; N = 1024 13.3 with 32, 14.0 with 64). With one pass of primes
+// N = 16384 has no clear line (64 and 128: 31 bits 13.8 and 17.0, 200 bits 17.6 and 15.8, 434 bits 20.5 and
+// 19.8, 450 bits 18.1 and 20.0). The table B has the 4 LW bytes of a coefficient sum and 4 bytes of the
+// quotient sum as columns; its accumulator takes a power of two of tensor-memory columns.
 constexpr int kCrt32Rows = 128;
 NC_HD constexpr int crt32_log_tile(int logN, int logN1) {
     const int t = logN >= 15 ? 7 : logN >= 12 ? 6 : 5;

@@ -45,13 +45,14 @@ void DeviceTables::check_stuck() const {
 namespace {
 std::mutex g_tables_mu;
 std::map<int, DeviceTables*> g_tables;
+// The devices' status words (Tables::stuck): kept until the process ends, since pinning one costs 2 ms.
+std::map<int, uint32_t*> g_stuck;
 
 void free_tables(DeviceTables* t) {
     for (void* ptr : {static_cast<void*>(t->fwd), static_cast<void*>(t->inv), static_cast<void*>(t->pow32),
                       static_cast<void*>(t->primes), static_cast<void*>(t->res_w), static_cast<void*>(t->fwd32),
                       static_cast<void*>(t->inv32), static_cast<void*>(t->pc32), static_cast<void*>(t->res_w32)})
         cudaFree(ptr);
-    cudaFreeHost(t->stuck);
 }
 
 // The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants and the residue stage's weight bytes (byte c of 2^(8 b) mod p_i at
@@ -99,7 +100,9 @@ DeviceTables* acquire_tables(int device) {
         check(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device), "device attribute");
         check(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, device), "device attribute");
         t->tensor_cores = NC_HAS_TCGEN05 && major == 10 && minor == 0;
-        check(cudaHostAlloc(&t->stuck, 64, cudaHostAllocMapped | cudaHostAllocPortable), "status word");
+        uint32_t*& word = g_stuck[device];
+        if (!word) check(cudaHostAlloc(&word, 64, cudaHostAllocMapped | cudaHostAllocPortable), "status word");
+        t->stuck = word;
         *t->stuck = 0;
         const size_t tw_bytes = size_t(kMaxPrimes) * kMaxN * sizeof(ulonglong2);
         check(cudaMalloc(&t->fwd, tw_bytes), "twiddle table");

@@ -756,16 +756,9 @@ std::string check_qconst32(const QConst32& c) {
     const int c0 = int(c.top_byte);
     if (c0 != std::max(0, (int(c.qbits) - 1) / 8 - 4)) return "first byte of the quotient's window";
     if (8 * c0 + c.top_shift + 14 != int(c.qbits)) return "shift of the quotient's window";
-    Big window = neg;  // floor(((-M) mod q) / 2^(8 c0))
-    Big byte{256};
-    for (int b = 0; b < c0; ++b) {
-        Big up;
-        divmod(window, byte, &up);
-        window = up;
-    }
-    window.resize(std::max<size_t>(window.size(), 2), 0);
-    if (window.size() != 2 || ((uint64_t(window[1]) << 32) | window[0]) != c.top_neg_m)
-        return "(-M) mod q in the quotient's window";
+    u128 window = 0;  // floor(((-M) mod q) / 2^(8 c0)), below 2^40
+    for (int w = kMqStride - 1; w >= c0 / 4; --w) window = (window << 32) | c.neg_m[w];
+    if (window >> (8 * (c0 % 4)) != c.top_neg_m) return "(-M) mod q in the quotient's window";
     return std::string();
 }
 

@@ -61,7 +61,7 @@ const std::vector<PrimeConst32>& prime_set32();
 // Primes of the 30-bit set for the bound of primes_needed (pairs only); -1 if more than 64.
 int primes_needed32(int logN, int qbits);
 
-// The 30-bit engine's CRT + Barrett constants. Returns an empty string or an error message.
+// The 30-bit engine's CRT constants. Returns an empty string or an error message.
 std::string build_qconst32(const uint32_t* q, int L, int logN, QConst32* out);
 
 // Table B of the 30-bit engine's tensor-core CRT in the MMA's shared-memory order. K byte 4 i + a

@@ -1,6 +1,6 @@
 // Kernels of the 30-bit word engine (w32.cuh): k_dec_tc32 (residues on the tensor cores + forward
 // column stages), k_row32 (row blocks) and k_crt_tc32 (inverse column stages + CRT on the tensor
-// cores + Barrett), with their launchers.
+// cores), with their launchers.
 //
 // Residues. With x_n given as 4 L bytes x_{n,b}, x_n mod p_i = sum_c 2^(8 c) S[n][i,c] with
 // S[n][i,c] = sum_b x_{n,b} w_{i,b,c}, w_{i,b,c} byte c (of 4) of 2^(8 b) mod p_i: the same u8 x u8
@@ -49,8 +49,8 @@ __device__ __forceinline__ uint64_t mad_wide(uint32_t a, uint32_t b, uint64_t c)
     return d;
 }
 
-// sum_c 2^(8 c) s[c] mod p into [0, 3.3 p) (the butterflies take [0, 4p)), for s[c] < 2^23 and p in
-// (2^29.8, 2^30): with lo = s0 + 2^8 s1 and hi = s2 + 2^8 s3 (both below 2^31.01), V = lo + 2^16 hi and
+// sum_c 2^(8 c) s[c] mod p into [0, 3.9 p) (the butterflies take [0, 4p)), for s[c] < 2^23 and p in
+// (7/8 2^30, 2^30): with lo = s0 + 2^8 s1 and hi = s2 + 2^8 s3 (both below 2^31.01), V = lo + 2^16 hi and
 // q = floor(hi floor(2^48 / p) / 2^32) falls short of 2^16 hi / p by less than 1 + hi / 2^32 < 1.6, and
 // lo < 2.3 p is not reduced: V - q p < 3.9 p. Five instructions, one of them a multiply-high (a 48-bit
 // sum and its Barrett quotient took ten).
@@ -767,7 +767,8 @@ __global__ void __launch_bounds__(kThreads, 4) k_crt_tc32(ProductDesc d, Tables 
 // for the staged twiddles and residues and for the other warps of a block. N = 65536, 868 bits,
 // blocks of 4096: 47.3 -> 44.8 us (padded places, block barriers, additions off the multiply pipe).
 // Resident CTAs per SM: radix-8 passes in 256-thread CTAs at four (64 registers: three and five CTAs
-// are no faster at N = 2^16), radix 16 at three.
+// are no faster at N = 2^16); radix 16 at two, which is what its shared memory (100 KB) lets in (its
+// launch bound of three holds it to 80 registers).
 template <int LOG_N2, int LOG_E, int THREADS>
 __global__ void __launch_bounds__(THREADS, (THREADS == 256 ? (LOG_E == 3 ? 4 : 3) : 2)) k_row32(ProductDesc d, Tables t,
                                                                                                    int early) {
