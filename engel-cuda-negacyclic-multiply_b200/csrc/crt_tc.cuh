@@ -202,8 +202,8 @@ __device__ bool crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
     }
     const uint32_t kq = uint32_t((frac + (1ull << 31)) >> 32);
 
-    // one warp polls, the others wait at the barrier
-    if (!__syncthreads_and(warp != 0 || bar_wait(t, crt_tc_detail::smem_u32(bar), parity, kGiveUpMmas) ? 1 : 0)) return false;
+    // (every thread waits for itself; whether all the waits ended well is seen at the next barrier)
+    const bool ok = bar_wait(t, crt_tc_detail::smem_u32(bar), parity, kGiveUpMmas);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t acc[W];
 #pragma unroll
@@ -245,7 +245,7 @@ __device__ bool crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
 
     // every thread is past its reads of A and of tensor memory: stage the tile's output in A
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (!__syncthreads_and(ok ? 1 : 0)) return false;
     uint32_t* s_out = reinterpret_cast<uint32_t*>(sA);
     if (tc < T) {
         uint32_t* o = s_out + tc * L;
