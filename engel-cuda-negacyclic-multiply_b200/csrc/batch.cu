@@ -176,7 +176,6 @@ void Batch::finalize(cudaStream_t stream) {
             dw.a_hat = e.a_hat;
             dw.hat_out = e.hat_out;
             bp.d = dw;
-            bp.tiles = uint32_t(g32.tiles);
             // operands with a residue stage: both (product), a (forward) or b (cached a)
             bp.first_operand = e.mode == kModeCachedA ? 1u : 0u;
             const uint32_t operands = e.mode == kModeProduct ? 2u : 1u;

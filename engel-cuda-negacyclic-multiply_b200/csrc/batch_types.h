@@ -29,7 +29,7 @@ struct BatchProduct {
     ProductDesc d;
     uint32_t n_dec;          // residue items of this product
     uint32_t n_row;          // row items
-    uint32_t tiles;          // residue tiles per operand
+    uint32_t tiles;          // 256-coefficient tiles per operand (62-bit engine)
     uint32_t first_operand;  // 1 when a is given in the NTT domain (only b is decomposed)
     uint32_t tiles_tc;       // 128-coefficient tiles per operand (residues on the tensor cores)
     uint32_t pad;

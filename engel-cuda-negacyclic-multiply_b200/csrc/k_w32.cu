@@ -349,7 +349,7 @@ __device__ __forceinline__ void dec_tc32_any(const ProductDesc& d, const Tables&
 
 // What bounds it: issue slots (the five-instruction fold of every residue, the column butterflies)
 // and the latency of a tile's phases, which four CTAs an SM overlap in part; DRAM and the tensor cores
-// are idle most of the time. Two operands of N = 65536, 868 bits: 34.8 -> 26.1 us (a fold of five
+// are idle most of the time. Two operands of N = 65536, 868 bits: 34.8 -> 25.9 us (a fold of five
 // instructions, neighbouring columns a thread, one polling warp, one bulk copy of
 // the weights).
 //
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_dec_tc32(ProductDesc d, Tables 
 // What bounds it: the column butterflies and loads (59 residues of a coefficient against one
 // contraction row), so integer issue and load latency, not the tensor cores. 128-coefficient tiles
 // with the primes in passes of 32 through one 20 KB A buffer keep a CTA at 54 KB, four per SM.
-// N = 65536, 868 bits: 24.6 -> 20.5 us a stage; N = 1024, where the old CRT was a chain of 59 dependent
+// N = 65536, 868 bits: 24.6 -> 19.7 us a stage; N = 1024, where the old CRT was a chain of 59 dependent
 // loads a thread in four CTAs: 32.8 -> 16.0 us a product.
 
 // A: [16 row groups][8 K chunks of four primes][8 rows][16 B], the chunks 16 or 32 bytes and the row
