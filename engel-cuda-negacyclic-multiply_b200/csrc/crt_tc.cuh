@@ -202,13 +202,14 @@ __device__ bool crt_coeffs_tc(const ProductDesc& d, const Tables& t, int tile, u
     }
     const uint32_t kq = uint32_t((frac + (1ull << 31)) >> 32);
 
-    // (every thread waits for itself; whether all the waits ended well is seen at the next barrier)
-    const bool ok = bar_wait(t, crt_tc_detail::smem_u32(bar), parity, kGiveUpMmas);
+    // (every warp waits for itself, and is together again for the reads of tensor memory; whether all the
+    // waits ended well is seen at the next barrier)
+    const bool ok = __all_sync(0xffffffffu, bar_wait(t, crt_tc_detail::smem_u32(bar), parity, kGiveUpMmas)) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t acc[W];
 #pragma unroll
     for (int w = 0; w < W; ++w) acc[w] = 0;
-    {
+    if (ok) {
         // fold S_c 2^(8c) into 32-bit words: two words per group of eight columns, one carry pass
         const uint32_t lane_base = taddr + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(half) * kHalfCol;
         uint64_t carry = 0;

@@ -55,8 +55,9 @@ void free_tables(DeviceTables* t) {
         cudaFree(ptr);
 }
 
-// The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants and the residue stage's weight bytes (byte c of 2^(8 b) mod p_i at
-// [i / 2][b / 16][4 (i % 2) + c][b % 16], b < 128: the MMA's B rows of a prime pair).
+// The 30-bit engine's tables: twiddles (w, floor(w 2^32 / p)), prime constants and the residue stage's
+// weight bytes (byte c of 2^(8 b) mod p_i at [i / 2][b / 16][4 (i % 2) + c][b % 16], b < 128: the MMA's B
+// rows of a prime pair).
 void upload_tables32(DeviceTables* t) {
     const HostTables32& h = host_tables32();
     const size_t tw = size_t(kMaxPrimes32) * kMaxN * sizeof(uint2);

@@ -12,9 +12,8 @@
 // accumulation in tensor memory is exact. The primes (any count up to 48) go through
 // tcgen05.mma kind::i8 in passes of 16 (128 accumulator columns); after each pass the eight warps
 // read the partial sums back (tcgen05.ld) and fold sum_c 2^(8 c) S_c (< 2^80) into [0, 2p) modulo p_i.
-// The tile is
-// C = 128 / N1 columns of all N1 rows of the polynomial (row length N2 = N / N1), as in k_dec, so
-// the forward column stages and the residue-row stores follow unchanged.
+// The tile is C = 128 / N1 columns of all N1 rows of the polynomial (row length N2 = N / N1), as in
+// k_dec, so the forward column stages and the residue-row stores follow unchanged.
 //
 // Operand bytes reach shared memory by cp.async, the weights by one bulk copy (no register staging).
 // Each prime's residues overwrite its own 1 KB of weights once its pass's MMAs have completed. A bounded
@@ -156,10 +155,11 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
     // and half w / 4 of the pass's primes
     const int m = 32 * (warp & 3) + lane;
     const int half = warp >> 2;
-    for (int g = 0; ok && g * kDecTcPassPrimes < k; ++g) {
+    bool failed = !ok;
+    for (int g = 0; g * kDecTcPassPrimes < k; ++g) {
         const int i0 = g * kDecTcPassPrimes;
         const int np = k - i0 < kDecTcPassPrimes ? k - i0 : kDecTcPassPrimes;
-        if (tid == 0) {
+        if (tid == 0 && !failed) {
             // kind::i8: D s32 (bits 4-5 = 2), A and B u8, K-major; N >> 3 at bit 17, M >> 4 at bit 24
             const uint32_t ng = uint32_t((np + 1) & ~1);
             const uint32_t idesc = (2u << 4) | (ng << 17) | (uint32_t(kDecTcRows >> 4) << 24);
@@ -178,7 +178,7 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
                          : "memory");
         }
         // one warp polls, the others wait at the barrier
-        ok = __syncthreads_and(warp != 0 || bar_wait(t, smem_u32(&bar), uint32_t(g & 1), kGiveUpMmas) ? 1 : 0) != 0;
+        ok = __syncthreads_and(warp != 0 || (!failed && bar_wait(t, smem_u32(&bar), uint32_t(g & 1), kGiveUpMmas)) ? 1 : 0) != 0;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int ib = i0 + 8 * half;
         const int ie = i0 + np < ib + 8 ? i0 + np : ib + 8;
@@ -201,12 +201,13 @@ __device__ __forceinline__ void dec_tc_item(const ProductDesc& d, const Tables& 
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        failed = !ok;
         __syncthreads();  // this pass's reads are done before the next MMA
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(kDecTcCols) : "memory");
-    if (!ok) {
+    if (failed) {
         report_stuck(t);
         return;
     }
